@@ -9,7 +9,9 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libmm_b200.so")
-SOURCES = ["conv.cu", "mixed.cu", "rhs.cu", "demag_setup.cu", "plan.cu", "compat.cu", "noalloc.cu", "io.cpp", "am12.cu", "unet.cu"]
+SOURCES = ["conv.cu", "mixed.cu", "rhs.cu:5", "rhs.cu:4", "rhs.cu:3", "rhs.cu:2", "rhs.cu:1", "rhs.cu:0", "demag_setup.cu", "plan.cu", "compat.cu", "noalloc.cu", "io.cpp", "am12.cu", "unet.cu"]
+# "name:k" compiles name with -DMM_RHS_PART=k: the four-step epilogue's instances in parts, in
+# parallel (eight cores: 8 min 15 s as one unit -> 2 min 30 s)
 HEADERS = ["fft.cuh", "fft4.cuh", "mixed.cuh", "kernel_view.cuh", "pdl.cuh", "mm_internal.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -17,7 +19,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std
 
 
 def _inputs():
-    files = [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
+    files = [os.path.join(CSRC, s.split(":")[0]) for s in SOURCES]
     files += [os.path.join(CSRC, h) for h in HEADERS]
     files.append(os.path.join(HERE, "..", "include", "mm_b200.h"))
     files.append(os.path.join(HERE, "..", "include", "libmumax2_compat.h"))
@@ -39,11 +41,12 @@ def build(force=False, verbose=True):
     objs = []
     procs = []
     for s in SOURCES:
-        src = os.path.join(CSRC, s)
+        name, _, part = s.partition(":")
+        src = os.path.join(CSRC, name)
         if not os.path.exists(src):
             continue
-        obj = os.path.join(objdir, s + ".o")
-        cmd = [NVCC] + FLAGS + ["-c", src, "-o", obj]
+        obj = os.path.join(objdir, name + part + ".o")
+        cmd = [NVCC] + FLAGS + (["-DMM_RHS_PART=" + part] if part else []) + ["-c", src, "-o", obj]
         procs.append((cmd, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT)))
         objs.append(obj)
     for cmd, p in procs:

@@ -13,6 +13,7 @@
 // estimate and the max-torque reduction.  The reference runs these as separate
 // kernels with a host sync after each (libmumax2.go), plus a D2H copy per reduction
 // (reductor.go:69-186).
+#include <algorithm>
 #include <cstdio>
 
 #include "fft.cuh"
@@ -21,6 +22,10 @@
 #include "mm_internal.h"
 #include "kernel_view.cuh"
 #include "pdl.cuh"
+
+#ifndef MM_RHS_PART
+#define MM_RHS_PART 0
+#endif
 
 namespace mm {
 using namespace mmfft;
@@ -401,7 +406,7 @@ __device__ __forceinline__ void energy_acc(const FieldParams& P, long long i, fl
 }
 
 // Block-level reduction of ThreadRed; thread 0 publishes.
-__device__ void block_reduce_publish(ThreadRed tr, const StageOp& op, DevCtl* ctl, unsigned int* tq_out, float* red) {
+static __device__ void block_reduce_publish(ThreadRed tr, const StageOp& op, DevCtl* ctl, unsigned int* tq_out, float* red) {
     __shared__ float s_tq[32], s_err[32];
     __shared__ int s_bad[32];
     __shared__ float s_e[32][8];
@@ -515,7 +520,7 @@ __device__ __forceinline__ void epilogue_cells_begin(const EpiArgs& A, const Dev
 
 // PointwiseUpdater.Update (update_pointwise.go:30-88): first row with time >= t, linear
 // interpolation from the row before; 0 at or before the first row; false past the last.
-__device__ bool table_value(const FieldParams::TimeTable& T, double t, double out[3]) {
+static __device__ bool table_value(const FieldParams::TimeTable& T, double t, double out[3]) {
     int i = 0;
     while (i < T.n && T.rows[4 * i] < t) i++;
     if (i >= T.n) return false;
@@ -533,7 +538,7 @@ __device__ bool table_value(const FieldParams::TimeTable& T, double t, double ou
 // The block's simulation scalars for the staged (shared-memory) variants: the
 // simulation's entry, with B_ext and j from their time tables at this evaluation's time.
 // Called by one thread.
-__device__ void stage_scalars(const EpiArgs& A, const DevCtl* ctl, SimScalars& s) {
+static __device__ void stage_scalars(const EpiArgs& A, const DevCtl* ctl, SimScalars& s) {
     s = A.P.sims ? A.P.sims[blockIdx.y] : A.P.s;
     if (A.P.tab[0].n || A.P.tab[1].n) {
         const double t = ctl ? ctl->t + A.op.c_time * ctl->dt : A.t_eval;
@@ -658,13 +663,39 @@ __host__ __device__ constexpr int xinv4_rpb() {
     return (384 / (3 * FS<M>::P2)) > 0 ? 384 / (3 * FS<M>::P2) : 1;
 }
 
-// Rows per block of the four-step epilogue: the default, or half of it (the autotuner's
-// other variant; at least 32 threads).  A compile-time constant, so that the row loops
-// of the epilogue unroll and its register budget stays that of a fixed tile.
-template <int M, bool HALF>
-__host__ __device__ constexpr int xinv4_rows_c() {
-    return (HALF && xinv4_rpb<M>() >= 2 && (xinv4_rpb<M>() / 2) * 3 * FS<M>::P2 >= 32) ? xinv4_rpb<M>() / 2
-                                                                                          : xinv4_rpb<M>();
+// Rows and threads per block of the row-shaped passes (C2R + epilogue, stage combine).  A
+// full tile (FLEX = false) is xinv4_rpb rows, a compile-time constant.  A FLEX launch passes
+// its own rows and may have more threads than the row transforms use: the extra ones work on
+// the cells only.
+//  * Grids that fill the GPU with full tiles: the full tile, or half of it (tile -1).
+//    (1024 rows of 1024 cells, 256 full tiles: in finer ones the torque takes 279 us, not 264.)
+//  * Fewer full tiles than SMs: the block's cells, not bandwidth, set the time (a
+//    192-thread block of 8 rows of 128 cells walks 5 cells per thread, one dependent
+//    round trip after the other), so the rows spread over up to two blocks per SM with a
+//    thread per cell (at most 384), at least 128 cells to a block while that leaves one
+//    block per SM.  tile -1: half as many rows.  RK45 step, before and after: 128x128 disk
+//    under Slonczewski torque 268 -> 148 us, 128x32 film 154 -> 107, 512x128 strip 214 -> 157.
+// The row count changes the block decomposition only; every cell's arithmetic is the same.
+struct RowTile {
+    bool flex;
+    int rpb, threads;
+};
+template <int M>
+static RowTile xinv4_shape(int nrows, int n2, int nsim, int tile) {
+    constexpr int R0 = xinv4_rpb<M>(), TR = 3 * FS<M>::P2, SMS = 148;
+    auto up32 = [](long long v) { return (int)((v + 31) / 32 * 32); };
+    const long long rows = (long long)nrows * nsim;
+    if ((long long)((nrows + R0 - 1) / R0) * nsim >= SMS) {
+        if (tile < 0 && R0 >= 2 && (R0 / 2) * TR >= 32) return {true, R0 / 2, up32((R0 / 2) * TR)};
+        return {false, R0, up32(R0 * TR)};
+    }
+    long long rpb = rows / (2 * SMS);
+    const long long fill = std::min<long long>((127 + n2) / n2, rows / SMS);
+    rpb = std::max(rpb, fill);
+    if (tile < 0) rpb /= 2;
+    rpb = std::min<long long>(std::max<long long>(rpb, 1), R0);
+    const long long cells = rpb * n2, turns = (cells + 383) / 384;
+    return {true, (int)rpb, std::max(up32((cells + turns - 1) / turns), up32(rpb * TR))};
 }
 
 // R2C rows from the block's shared-memory lines: float x of the line of (row, c) holds the
@@ -755,11 +786,11 @@ __device__ __forceinline__ void prefetch_epilogue_rows(const EpiArgs& A, int row
         if (j != op.ecur) streams3(op.ep[j].get(cur));
 }
 
-template <int M, bool TERMS, bool BATCH, bool HALF, bool FWD, int SPEC>
+template <int M, bool TERMS, bool BATCH, bool FLEX, bool FWD, int SPEC>
 __device__ __forceinline__ void xinv4_epi_body(typename SpecIn<FWD>::type S, int hp, int L1,
-                                               const float2* __restrict__ tw, const EpiArgs& A) {
+                                               const float2* __restrict__ tw, const EpiArgs& A, int rpb) {
     pdl_begin();
-    constexpr int RPB = xinv4_rows_c<M, HALF>();
+    const int RPB = FLEX ? rpb : xinv4_rpb<M>();
     const DevCtl* ctl = A.ctl ? A.ctl + blockIdx.y : nullptr;
     if (skip_eval(ctl, A.skip_retry)) return;
     S += blockIdx.y * A.spec_bstride;
@@ -827,41 +858,40 @@ __device__ __forceinline__ void xinv4_epi_body(typename SpecIn<FWD>::type S, int
 // (78-80 registers; the SPEC_LEAN epilogue 56-69); batched plans: two blocks per SM requested
 // explicitly (their staged-scalar variant would otherwise take 136-150 registers and one
 // block).
-template <int M, bool TERMS, bool HALF, bool FWD, int SPEC>
+template <int M, bool TERMS, bool FLEX, bool FWD, int SPEC>
 __global__ void __launch_bounds__(384) xinv4_epi_kernel(typename SpecIn<FWD>::type S, int hp, int L1,
-                                                        const float2* __restrict__ tw, EpiArgs A) {
-    xinv4_epi_body<M, TERMS, false, HALF, FWD, SPEC>(S, hp, L1, tw, A);
+                                                        const float2* __restrict__ tw, EpiArgs A, int rpb) {
+    xinv4_epi_body<M, TERMS, false, FLEX, FWD, SPEC>(S, hp, L1, tw, A, rpb);
 }
 
 // The SPEC_LEAN epilogue without the next stage's rows fits 56 registers: three blocks per SM
 // requested (RK23 film step 478 -> 476 us; the variant that writes the rows spills at 56
 // and keeps the kernel above, two blocks per SM).
-template <int M, bool HALF>
+template <int M, bool FLEX>
 __global__ void __launch_bounds__(384, 3) xinv4_epi_lean3_kernel(const float2* __restrict__ S, int hp, int L1,
-                                                                 const float2* __restrict__ tw, EpiArgs A) {
-    xinv4_epi_body<M, false, false, HALF, false, SPEC_LEAN>(S, hp, L1, tw, A);
+                                                                 const float2* __restrict__ tw, EpiArgs A, int rpb) {
+    xinv4_epi_body<M, false, false, FLEX, false, SPEC_LEAN>(S, hp, L1, tw, A, rpb);
 }
 
-template <int M, bool TERMS, bool HALF, bool FWD, int SPEC>
+template <int M, bool TERMS, bool FLEX, bool FWD, int SPEC>
 __global__ void __launch_bounds__(384, M <= 512 ? 2 : 1) xinv4_epi_batch_kernel(typename SpecIn<FWD>::type S,
                                                                                 int hp, int L1,
                                                                                 const float2* __restrict__ tw,
-                                                                                EpiArgs A) {
-    xinv4_epi_body<M, TERMS, true, HALF, FWD, SPEC>(S, hp, L1, tw, A);
+                                                                                EpiArgs A, int rpb) {
+    xinv4_epi_body<M, TERMS, true, FLEX, FWD, SPEC>(S, hp, L1, tw, A, rpb);
 }
 
 // ---------------------------------------------------------------- stage combine + R2C rows
 // The first stage state of an attempt, formed as combine_kernel forms it (same operations
 // in the same order), written to A.next and, times the Msat mask when fwd_mask, turned
 // into its R2C rows in the spectrum: the attempt's first evaluation then starts at its
-// column pass.  Blocks and threads as the four-step C2R + epilogue pass: RPB rows (z, y)
-// per block, P2 threads per (row, component) line.
+// column pass.  Blocks and threads as the four-step C2R + epilogue pass (xinv4_shape): RPB
+// rows (z, y) per block, P2 threads per (row, component) line.
 template <int M>
 __global__ void __launch_bounds__(384) combine_rows_kernel(CombineArgs A, int n0, int n1, int n2, float2* S, int hp,
                                                            int L1, long long spec_bstride,
-                                                           const float2* __restrict__ tw, int fwd_mask) {
+                                                           const float2* __restrict__ tw, int fwd_mask, int RPB) {
     pdl_begin();
-    constexpr int RPB = xinv4_rows_c<M, false>();
     using F = FS<M>;
     const DevCtl* ctl = A.ctl + blockIdx.y;
     if (ctl->done) return;
@@ -927,11 +957,29 @@ __global__ void __launch_bounds__(384) combine_rows_kernel(CombineArgs A, int n0
     r2c_staged_lines<M>(v, buf, twt, tw, t, active, n2, dst);
 }
 
+// What the evaluation lacks, as SPEC_* bits: no per-cell mask of any kind, no thermal
+// term, no Zhang-Li or Slonczewski term.
+static int epilogue_spec(const FieldParams& P) {
+    int spec = SPEC_NOMASK;
+    if (!P.thermal) spec |= SPEC_NOTHERMAL;
+    if (!P.zhangli && !P.slonczewski) spec |= SPEC_NOSTT;
+    const float* masks[] = {P.msat_mask,      P.aex_mask,      P.alpha_mask,     P.ku_mask,        P.anisu_mask[0],
+                            P.anisu_mask[1],  P.anisu_mask[2], P.bext_mask[0],   P.bext_mask[1],   P.bext_mask[2],
+                            P.j_mask[0],      P.j_mask[1],     P.j_mask[2],      P.temp_mask,      P.xi_mask,
+                            P.zl_pol_mask,    P.p_mask[0],     P.p_mask[1],      P.p_mask[2],      P.sl_pol_mask,
+                            P.lambda_mask,    P.eps_prime_mask, P.t_fl_mask};
+    for (const float* q : masks)
+        if (q) spec &= ~SPEC_NOMASK;
+    return spec;
+}
+
+#if MM_RHS_PART == 0
 template <int M>
 static cudaError_t launch_combine_rows_t(const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
                                          long long spec_bstride, const float2* tw, int fwd_mask, int nsim,
                                          cudaStream_t st) {
-    constexpr int RPB = xinv4_rows_c<M, false>();
+    const RowTile tile = xinv4_shape<M>(n[0] * n[1], n[2], nsim, 0);
+    const int RPB = tile.rpb, threads = tile.threads;
     const size_t smem = (size_t)(RPB * 3 * FS<M>::LBUF + FS<M>::TWT + M / 2 + 1) * sizeof(float2);
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(combine_rows_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -939,10 +987,8 @@ static cudaError_t launch_combine_rows_t(const CombineArgs& A, const int n[3], f
         if (e != cudaSuccess) return e;
     }
     const int blocks = (n[0] * n[1] + RPB - 1) / RPB;
-    int threads = RPB * 3 * FS<M>::P2;
-    if (threads < 32) threads = 32;
     return launch_pdl(combine_rows_kernel<M>, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, A, n[0],
-                      n[1], n[2], S, hp, L1, spec_bstride, tw, fwd_mask);
+                      n[1], n[2], S, hp, L1, spec_bstride, tw, fwd_mask, RPB);
 }
 
 cudaError_t launch_combine_rows(int M, const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
@@ -1240,22 +1286,6 @@ static cudaError_t launch_xinv_t(const float2* S, int hp, int L1, const float2* 
     return cudaGetLastError();
 }
 
-// What the evaluation lacks, as SPEC_* bits: no per-cell mask of any kind, no thermal
-// term, no Zhang-Li or Slonczewski term.
-static int epilogue_spec(const FieldParams& P) {
-    int spec = SPEC_NOMASK;
-    if (!P.thermal) spec |= SPEC_NOTHERMAL;
-    if (!P.zhangli && !P.slonczewski) spec |= SPEC_NOSTT;
-    const float* masks[] = {P.msat_mask,      P.aex_mask,      P.alpha_mask,     P.ku_mask,        P.anisu_mask[0],
-                            P.anisu_mask[1],  P.anisu_mask[2], P.bext_mask[0],   P.bext_mask[1],   P.bext_mask[2],
-                            P.j_mask[0],      P.j_mask[1],     P.j_mask[2],      P.temp_mask,      P.xi_mask,
-                            P.zl_pol_mask,    P.p_mask[0],     P.p_mask[1],      P.p_mask[2],      P.sl_pol_mask,
-                            P.lambda_mask,    P.eps_prime_mask, P.t_fl_mask};
-    for (const float* q : masks)
-        if (q) spec &= ~SPEC_NOMASK;
-    return spec;
-}
-
 // ---------------------------------------------------------------- mixed-radix C2R + epilogue
 // Row lengths M that are not powers of two: the pre-processing of xinv_epi_kernel, the
 // mixed-radix inverse transform of mixed.cuh, then the same epilogue.  rpb rows of three
@@ -1347,37 +1377,34 @@ static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, cons
     return cudaGetLastError();
 }
 
-template <int M>
-static int xinv4_rows(int tile) {
-    return tile < 0 ? xinv4_rows_c<M, true>() : xinv4_rows_c<M, false>();
-}
+#endif  // MM_RHS_PART == 0
 
-template <int M, bool TERMS, bool BATCH, bool HALF, bool FWD>
+template <int M, bool TERMS, bool BATCH, bool FLEX, bool FWD>
 static cudaError_t launch_xinv4_h(const float2* S, int hp, int L1, const float2* tw, const EpiArgs& A,
-                                  cudaStream_t st, int* nblocks, int nsim) {
-    constexpr int RPB = xinv4_rows_c<M, HALF>();
+                                  cudaStream_t st, int* nblocks, int nsim, const RowTile& tile) {
+    const int RPB = tile.rpb, threads = tile.threads;
     const size_t smem = (size_t)(RPB * 3 * FS<M>::LBUF + FS<M>::TWT + (FWD ? M / 2 + 1 : 0)) * sizeof(float2);
     // Single plans: the SPEC_LEAN kernels when nothing of the three is present, else the
     // kernel without what is absent of masks and thermal (see below), else the general one.  Batched plans: without thermal and spin-transfer terms (relaxation
     // pools, masks kept) or without masks and spin-transfer terms (thermal ensembles).
     const int spec = TERMS ? 0 : epilogue_spec(A.P);
-    auto kern = xinv4_epi_kernel<M, TERMS, HALF, FWD, 0>;
+    auto kern = xinv4_epi_kernel<M, TERMS, FLEX, FWD, 0>;
     if (BATCH) {
         constexpr int NOTS = SPEC_NOTHERMAL | SPEC_NOSTT, NOMS = SPEC_NOMASK | SPEC_NOSTT;
-        kern = xinv4_epi_batch_kernel<M, TERMS, HALF, FWD, 0>;
+        kern = xinv4_epi_batch_kernel<M, TERMS, FLEX, FWD, 0>;
         if constexpr (!TERMS) {
-            if ((spec & NOTS) == NOTS) kern = xinv4_epi_batch_kernel<M, false, HALF, FWD, NOTS>;
-            else if ((spec & NOMS) == NOMS) kern = xinv4_epi_batch_kernel<M, false, HALF, FWD, NOMS>;
+            if ((spec & NOTS) == NOTS) kern = xinv4_epi_batch_kernel<M, false, FLEX, FWD, NOTS>;
+            else if ((spec & NOMS) == NOMS) kern = xinv4_epi_batch_kernel<M, false, FLEX, FWD, NOMS>;
         }
     } else if (spec == SPEC_LEAN) {
-        if constexpr (FWD) kern = xinv4_epi_kernel<M, false, HALF, true, SPEC_LEAN>;
-        else kern = xinv4_epi_lean3_kernel<M, HALF>;
+        if constexpr (FWD) kern = xinv4_epi_kernel<M, false, FLEX, true, SPEC_LEAN>;
+        else kern = xinv4_epi_lean3_kernel<M, FLEX>;
     } else if constexpr (!TERMS) {
         // masked films without thermal and spin-transfer terms; unmasked ones with a
         // spin-transfer term and no thermal one (the Neel wall under current)
         constexpr int NOTS = SPEC_NOTHERMAL | SPEC_NOSTT, NOMT = SPEC_NOMASK | SPEC_NOTHERMAL;
-        if ((spec & NOTS) == NOTS) kern = xinv4_epi_kernel<M, false, HALF, FWD, NOTS>;
-        else if ((spec & NOMT) == NOMT) kern = xinv4_epi_kernel<M, false, HALF, FWD, NOMT>;
+        if ((spec & NOTS) == NOTS) kern = xinv4_epi_kernel<M, false, FLEX, FWD, NOTS>;
+        else if ((spec & NOMT) == NOMT) kern = xinv4_epi_kernel<M, false, FLEX, FWD, NOMT>;
     }
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1393,18 +1420,16 @@ static cudaError_t launch_xinv4_h(const float2* S, int hp, int L1, const float2*
     }
     const int nrows = A.P.n[0] * A.P.n[1];
     const int blocks = (nrows + RPB - 1) / RPB;
-    int threads = RPB * 3 * FS<M>::P2;
-    if (threads < 32) threads = 32;
     *nblocks = blocks;
-    return launch_pdl(kern, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, S, hp, L1, tw, A);
+    return launch_pdl(kern, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, S, hp, L1, tw, A, RPB);
 }
 
 template <int M, bool TERMS, bool BATCH, bool FWD>
 static cudaError_t launch_xinv4_f(const float2* S, int hp, int L1, const float2* tw, const EpiArgs& A,
                                   cudaStream_t st, int* nblocks, int nsim, int tile) {
-    if (tile < 0 && xinv4_rows_c<M, true>() != xinv4_rows_c<M, false>())
-        return launch_xinv4_h<M, TERMS, BATCH, true, FWD>(S, hp, L1, tw, A, st, nblocks, nsim);
-    return launch_xinv4_h<M, TERMS, BATCH, false, FWD>(S, hp, L1, tw, A, st, nblocks, nsim);
+    const RowTile shape = xinv4_shape<M>(A.P.n[0] * A.P.n[1], A.P.n[2], nsim, tile);
+    if (shape.flex) return launch_xinv4_h<M, TERMS, BATCH, true, FWD>(S, hp, L1, tw, A, st, nblocks, nsim, shape);
+    return launch_xinv4_h<M, TERMS, BATCH, false, FWD>(S, hp, L1, tw, A, st, nblocks, nsim, shape);
 }
 
 // A.fwd selects the variant that also writes the R2C rows of the next stage state (no
@@ -1420,27 +1445,53 @@ static cudaError_t launch_xinv4_t(const float2* S, int hp, int L1, const float2*
     return launch_xinv4_f<M, TERMS, BATCH, false>(S, hp, L1, tw, A, st, nblocks, nsim, tile);
 }
 
+// The four-step pass of one row length, with or without per-term outputs and staged
+// scalars.  Its instances, most of this file's compile time, are spread over several
+// translation units (MM_RHS_PART, see build.py).
+template <int M>
+cudaError_t launch_xinv4(const float2* S, int hp, int L1, const float2* tw, const EpiArgs& A, bool terms, bool staged,
+                         cudaStream_t st, int* nblocks, int nsim, int tile)
+#if MM_RHS_PART > 0
+{
+    if (staged)
+        return terms ? launch_xinv4_t<M, true, true>(S, hp, L1, tw, A, st, nblocks, nsim, tile)
+                     : launch_xinv4_t<M, false, true>(S, hp, L1, tw, A, st, nblocks, nsim, tile);
+    return terms ? launch_xinv4_t<M, true, false>(S, hp, L1, tw, A, st, nblocks, 1, tile)
+                 : launch_xinv4_t<M, false, false>(S, hp, L1, tw, A, st, nblocks, 1, tile);
+}
+#define X(m)                                                                                                    \
+    template cudaError_t launch_xinv4<m>(const float2*, int, int, const float2*, const EpiArgs&, bool, bool,    \
+                                         cudaStream_t, int*, int, int);
+#if MM_RHS_PART == 1
+X(4) X(8) X(16)
+#elif MM_RHS_PART == 2
+X(32) X(64)
+#elif MM_RHS_PART == 3
+X(128) X(256)
+#elif MM_RHS_PART == 4
+X(512)
+#else
+X(1024)
+#endif
+#undef X
+#else
+;
+
 static bool use_xinv4(int M) { return M >= 4 && M <= 1024 && mr_pow2(M); }
 
 // The four-step epilogue (and the four-step row pass whose output it reproduces) serve
 // these row lengths.
 bool epi_r2c_supported(int M) { return use_xinv4(M); }
 
+// The most blocks per simulation that the pass may take for n0n1 rows (the size of the
+// reduction partials).
 int xinv_blocks(int M, int n0n1) {
     if (!mr_pow2(M)) {
         int rpb, nt;
         mr_xinv_shape(M, &rpb, &nt);
         return (n0n1 + rpb - 1) / rpb;
     }
-    if (use_xinv4(M)) {
-        int rpb = 1;
-        switch (M) {
-#define X(m) case m: rpb = xinv4_rows<m>(-1); break;
-            X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024)
-#undef X
-        }
-        return (n0n1 + rpb - 1) / rpb;
-    }
+    if (use_xinv4(M)) return n0n1;  // one row per block
     int TPL = mmfft::tpl(M);
     int rpb = (3 * TPL >= 384) ? 1 : 384 / (3 * TPL);
     size_t smem = (size_t)rpb * 3 * mmfft::line_len(M) * sizeof(float2);
@@ -1456,13 +1507,7 @@ cudaError_t launch_xinv_epi(int M, const float2* S, int hp, int L1, const float2
     const bool staged = staged_scalars(A, nsim);
     if (use_xinv4(M)) {
         switch (M) {
-#define X(m)                                                                      \
-    case m:                                                                       \
-        if (staged)                                                                     \
-            return terms ? launch_xinv4_t<m, true, true>(S, hp, L1, tw, A, st, nblocks, nsim, tile)  \
-                         : launch_xinv4_t<m, false, true>(S, hp, L1, tw, A, st, nblocks, nsim, tile); \
-        return terms ? launch_xinv4_t<m, true, false>(S, hp, L1, tw, A, st, nblocks, 1, tile)     \
-                     : launch_xinv4_t<m, false, false>(S, hp, L1, tw, A, st, nblocks, 1, tile);
+#define X(m) case m: return launch_xinv4<m>(S, hp, L1, tw, A, terms, staged, st, nblocks, nsim, tile);
             X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024)
 #undef X
         }
@@ -1508,5 +1553,6 @@ cudaError_t launch_local_epi(const EpiArgs& A, bool terms, cudaStream_t st, int*
     }
     return cudaGetLastError();
 }
+#endif  // MM_RHS_PART
 
 }  // namespace mm
