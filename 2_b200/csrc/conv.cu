@@ -23,7 +23,9 @@
 #include "fft4.cuh"
 #include "mm_internal.h"
 #include "kernel_view.cuh"
+#include "mixed.cuh"
 #include "pdl.cuh"
+#include "rdft.cuh"
 
 namespace mm {
 using namespace mmfft;
@@ -282,16 +284,18 @@ __global__ void colmul_kernel(float2* __restrict__ S, KernelView K, int ncols, l
 // transform is a length-P DFT held in registers.  The two halves of the inverse are
 // summed with one shuffle.  Replaces the z column FFT + multiply + inverse of colmul.
 
-// exp(SIGN 2 pi i z / (2P)) from the FP32 table
+// exp(SIGN 2 pi i m / (2P)), m < 2P, from an FP32 table in which it has stride tws (the
+// 4096-entry table, or for P that is not a power of two the table of length 2P)
 template <int SIGN>
-__device__ __forceinline__ float2 wtab(const float2* __restrict__ tw, int num, int den) {
-    return TwSrc<SIGN, float2>::get(tw, num, den);
+__device__ __forceinline__ float2 wtab(const float2* __restrict__ tw, int m, int tws) {
+    const float2 w = __ldg(tw + m * tws);
+    return SIGN > 0 ? make_float2(w.x, -w.y) : w;
 }
 
 template <int P, bool BATCH>
 __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, KernelView K, int L1, int h, int hp,
                                                        long long comp_stride, long long zstride, float scale,
-                                                       const float2* __restrict__ tw, const DevCtl* ctl,
+                                                       const float2* __restrict__ tw, int tws, const DevCtl* ctl,
                                                        int skip_retry, long long sim_stride,
                                                        const float* __restrict__ sim_scale) {
     pdl_begin();
@@ -318,7 +322,7 @@ __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, K
     if (s) {
 #pragma unroll
         for (int z = 1; z < P; z++) {
-            const float2 w = wtab<-1>(tw, z, 2 * P);
+            const float2 w = wtab<-1>(tw, z, tws);
 #pragma unroll
             for (int c = 0; c < 3; c++) x[c][z] = cmul(x[c][z], w);
         }
@@ -351,7 +355,7 @@ __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, K
     if (s) {
 #pragma unroll
         for (int z = 1; z < P; z++) {
-            const float2 w = wtab<+1>(tw, z, 2 * P);
+            const float2 w = wtab<+1>(tw, z, tws);
 #pragma unroll
             for (int c = 0; c < 3; c++) x[c][z] = cmul(x[c][z], w);
         }
@@ -364,7 +368,7 @@ __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, K
             float2 v = x[c][z];
             v.x += __shfl_xor_sync(0xffffffffu, v.x, 1);
             v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
-            const bool mine = (P == 1) ? (s == 0) : ((z < P / 2) == (s == 0));
+            const bool mine = (z < (P + 1) / 2) == (s == 0);
             if (active && mine) base[c * comp_stride + z * zstride] = v;
         }
 }
@@ -377,7 +381,7 @@ __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, K
 template <int P, bool BATCH>
 __global__ void __launch_bounds__(128) zmul_reg4_kernel(float2* __restrict__ S, KernelView K, int L1, int h, int hp,
                                                          long long comp_stride, long long zstride, float scale,
-                                                         const float2* __restrict__ tw, const DevCtl* ctl,
+                                                         const float2* __restrict__ tw, int tws, const DevCtl* ctl,
                                                          int skip_retry, long long sim_stride,
                                                          const float* __restrict__ sim_scale) {
     pdl_begin();
@@ -397,7 +401,7 @@ __global__ void __launch_bounds__(128) zmul_reg4_kernel(float2* __restrict__ S, 
     float2* base = S + (long long)ky * hp + kx;
     // W_{2P}^m, m < 2P, in shared memory (the lane-dependent twiddles below)
     __shared__ float2 wz[2 * P];
-    for (int m = threadIdx.x; m < 2 * P; m += blockDim.x) wz[m] = wtab<-1>(tw, m, 2 * P);
+    for (int m = threadIdx.x; m < 2 * P; m += blockDim.x) wz[m] = wtab<-1>(tw, m, tws);
     __syncthreads();
     float2 g[3][H];
     // forward: fold the P input planes onto P/2 with the lane's twiddles
@@ -480,41 +484,49 @@ __global__ void __launch_bounds__(128) zmul_reg4_kernel(float2* __restrict__ S, 
 
 template <int P>
 static cudaError_t launch_zmul_reg_t(float2* S, const KernelView& K, int L1, int h, int hp, long long comp_stride,
-                                     long long zstride, float scale, const float2* tw, const DevCtl* ctl,
-                                     int skip_retry, cudaStream_t st, int nsim, long long sim_stride,
-                                     const float* sim_scale) {
+                                     long long zstride, float scale, const float2* tw, int tws,
+                                     const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+                                     long long sim_stride, const float* sim_scale) {
     const long long threads = 2LL * L1 * h;
     const dim3 grid((unsigned)((threads + 127) / 128), (unsigned)nsim);
     if (nsim > 1)
         return launch_pdl(zmul_reg_kernel<P, true>, grid, dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride,
-                          scale, tw, ctl, skip_retry, sim_stride, sim_scale);
+                          scale, tw, tws, ctl, skip_retry, sim_stride, sim_scale);
     return launch_pdl(zmul_reg_kernel<P, false>, grid, dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride, scale,
-                      tw, ctl, skip_retry, sim_stride, sim_scale);
+                      tw, tws, ctl, skip_retry, sim_stride, sim_scale);
 }
 
 template <int P>
 static cudaError_t launch_zmul_reg4_t(float2* S, const KernelView& K, int L1, int h, int hp, long long comp_stride,
-                                      long long zstride, float scale, const float2* tw, const DevCtl* ctl,
-                                      int skip_retry, cudaStream_t st, int nsim, long long sim_stride,
-                                      const float* sim_scale) {
+                                      long long zstride, float scale, const float2* tw, int tws,
+                                      const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+                                      long long sim_stride, const float* sim_scale) {
     const long long threads = 4LL * L1 * h;
     const dim3 grid((unsigned)((threads + 127) / 128), (unsigned)nsim);
     if (nsim > 1)
         return launch_pdl(zmul_reg4_kernel<P, true>, grid, dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride,
-                          scale, tw, ctl, skip_retry, sim_stride, sim_scale);
+                          scale, tw, tws, ctl, skip_retry, sim_stride, sim_scale);
     return launch_pdl(zmul_reg4_kernel<P, false>, grid, dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride, scale,
-                      tw, ctl, skip_retry, sim_stride, sim_scale);
+                      tw, tws, ctl, skip_retry, sim_stride, sim_scale);
 }
 
-// P = N0 = L0/2 (zero-padded z); returns cudaErrorNotSupported for other shapes
+// P = N0 = L0/2 (zero-padded z), 1..16
 cudaError_t launch_zmul_reg(int P, float2* S, const KernelView& K, int L1, int h, int hp, long long comp_stride,
                             long long zstride, float scale, const float2* tw, const DevCtl* ctl, int skip_retry,
                             cudaStream_t st, int nsim, long long sim_stride, const float* sim_scale) {
+    int tws = TWN / (2 * P);
+    if (!mr_pow2(P)) {
+        tws = 1;
+        if (!mr_tables(2 * P, &tw, nullptr)) return cudaErrorInvalidValue;
+    }
     switch (P) {
-#define X(p, f) case p: return f<p>(S, K, L1, h, hp, comp_stride, zstride, scale, tw, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
-        // two lanes per column up to P = 8 (measured: P = 4, 128x128x4 ensemble class
+#define X(p, f) case p: return f<p>(S, K, L1, h, hp, comp_stride, zstride, scale, tw, tws, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
+        // two lanes per column up to P = 15 (measured: P = 4, 128x128x4 ensemble class
         // 1073 -> 1012 us; P = 8, 8x128x128 film 11.8 -> 11.0 us), four at P = 16
-        X(1, launch_zmul_reg_t) X(2, launch_zmul_reg_t) X(4, launch_zmul_reg_t) X(8, launch_zmul_reg_t)
+        X(1, launch_zmul_reg_t) X(2, launch_zmul_reg_t) X(3, launch_zmul_reg_t) X(4, launch_zmul_reg_t)
+        X(5, launch_zmul_reg_t) X(6, launch_zmul_reg_t) X(7, launch_zmul_reg_t) X(8, launch_zmul_reg_t)
+        X(9, launch_zmul_reg_t) X(10, launch_zmul_reg_t) X(11, launch_zmul_reg_t) X(12, launch_zmul_reg_t)
+        X(13, launch_zmul_reg_t) X(14, launch_zmul_reg_t) X(15, launch_zmul_reg_t)
         X(16, launch_zmul_reg4_t)
 #undef X
         default: return cudaErrorNotSupported;

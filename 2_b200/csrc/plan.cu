@@ -882,7 +882,7 @@ extern "C" MM_API long long mm_plan_device_bytes(mm_plan p) { return p ? p->byte
 // the register z-multiply applies when z is zero-padded (L0 = 2 N0) with N0 <= 16
 static bool zreg_ok(const ConvGeom& g) {
     const int n0 = g.n[0];
-    return g.L[0] == 2 * n0 && (n0 == 1 || n0 == 2 || n0 == 4 || n0 == 8 || n0 == 16);
+    return g.L[0] == 2 * n0 && n0 <= 16;
 }
 
 // ---------------------------------------------------------------- one evaluation

@@ -1,0 +1,24 @@
+"""The convolution passes at the sizes where their stages and tiles change: every length of
+the register z multiply; demag field and torque against the FP64 oracle."""
+import pytest
+
+from helpers import rand_m, rel_err, to_np
+
+pytestmark = pytest.mark.gpu
+
+Z_LENGTHS = [(n0, 4, 6) for n0 in range(2, 18)]       # 2..16 in registers, 17 in columns
+
+
+# FP32 transforms of L points accumulate about eps * log2(L) <= 12 * 6e-8 relative to the
+# largest field: 1e-6 bounds them, with the kernel's own rounding
+@pytest.mark.parametrize("n", Z_LENGTHS)
+def test_demag_and_torque_at_size(n):
+    import oracle as O
+    from mumax2 import Plan
+    prob = O.full_desc(n=n, cell=(3e-9, 4e-9, 5e-9), demag=1, exchange=1, msat=8e5, aex=1.3e-11, alpha=0.05,
+                       demag_accuracy=2)
+    o, g = O.Oracle(prob), Plan(prob)
+    m = rand_m(n, seed=sum(n))
+    assert rel_err(to_np(g.fields(m)["demag"]), o.fields(m)["demag"]) < 1e-6
+    assert rel_err(to_np(g.torque(m)[0]), o.torque(m)[0]) < 2e-6
+    g.close()
