@@ -1,0 +1,507 @@
+// colmix.cu -- column passes for any transform length with prime factors up to 31.
+//
+// A block holds TC adjacent kx columns in shared memory as [element][column], so every
+// access of a half-warp is to consecutive columns (no bank conflicts at any stride), all
+// lanes of a column group share their twiddles, and global rows move TC*8 contiguous bytes.
+//
+// Zero padding: with at most N = L/2 non-zero rows the length-L transform splits by the
+// parity of the frequency, X[2k] = DFT_N(x)[k] and X[2k+1] = DFT_N(x W_L^n)[k], and the
+// inverse's first N rows are the sum of the two length-N inverses (the odd one times
+// W_L^-n).  NP = 2 then; periodic axes have NP = 1, N = L.
+//
+// The length-N transform is in place with few, large radices (at most 16; 2-3 stages up to
+// N = 4096): the forward stages decimate in frequency and leave the frequencies in
+// digit-reversed slots, the inverse stages are their mirror images, so nothing is reordered
+// and the last forward stage, the kernel multiply and the first inverse stage work on the
+// same slots in registers (Gentleman & Sande 1966).  The first stage reads global memory and
+// the last one writes it: a 3x3 multiply of two-stage columns needs two barriers.
+#include <algorithm>
+
+#include "kernel_view.cuh"
+#include "mixed.cuh"
+#include "mm_internal.h"
+#include "pdl.cuh"
+#include "rdft.cuh"
+
+namespace mm {
+using namespace mmfft;
+
+constexpr int MC_MAXST = 12;
+
+struct ColPlan {
+    int N, NP, nst;
+    int r[MC_MAXST];  // radices in the order of the forward stages; the last one is the smallest
+    int nq;           // N / r[nst - 1]
+    int tws;          // W_L^m = tw[m * tws]
+    int sh;           // log2 of the columns per block (TC)
+};
+
+namespace {
+
+// a run-time radix 17..31 (prime): the paired sums of dft_prime on a local array, constants
+// from the twiddle table (W_R^m = tw[m * step])
+template <int SIGN>
+__device__ __noinline__ void dft_any(float2* a, int R, const float2* __restrict__ tw, int step) {
+    const int H = (R - 1) / 2;
+    float2 s[16], d[16];
+    float2 sum = a[0];
+    for (int n = 1; n <= H; n++) {
+        s[n] = cadd(a[n], a[R - n]);
+        d[n] = csub(a[n], a[R - n]);
+        sum = cadd(sum, s[n]);
+    }
+    const float2 a0 = a[0];
+    a[0] = sum;
+    for (int k = 1; k <= H; k++) {
+        float2 A = a0, B = make_float2(0.f, 0.f);
+        int m = 0;
+        for (int n = 1; n <= H; n++) {
+            m += k;
+            if (m >= R) m -= R;
+            const float2 w = tw[m * step];  // cos, -sin
+            A.x += w.x * s[n].x;
+            A.y += w.x * s[n].y;
+            B.x -= w.y * d[n].x;
+            B.y -= w.y * d[n].y;
+        }
+        const float2 iB = mul_si<SIGN>(B);
+        a[k] = cadd(A, iB);
+        a[R - k] = csub(A, iB);
+    }
+}
+
+// R = 0: the run-time radix `rad`
+template <int R, int SIGN>
+__device__ __forceinline__ void dft_r(float2* v, int rad, const ColPlan& P, const float2* __restrict__ tw) {
+    if constexpr (R > 0) RDft<R, SIGN>::run(v);
+    else dft_any<SIGN>(v, rad, tw, P.NP * P.N / rad * P.tws);
+}
+template <int R> struct RegLen { static constexpr int n = R > 0 ? R : 31; };
+
+template <int SIGN>
+__device__ __forceinline__ float2 tw_l(const ColPlan& P, const float2* __restrict__ tw, int m) {
+    const float2 w = __ldg(tw + m * P.tws);
+    return SIGN > 0 ? make_float2(w.x, -w.y) : w;
+}
+
+#define MC_EACH(r, rad) _Pragma("unroll") for (int r = 0; r < (R > 0 ? R : rad); r++)
+#define MC_SWITCH(rad, CALL)                                                                                   \
+    switch (rad) {                                                                                             \
+        case 1: CALL(1); break;                                                                                \
+        case 2: CALL(2); break;                                                                                \
+        case 3: CALL(3); break;                                                                                \
+        case 4: CALL(4); break;                                                                                \
+        case 5: CALL(5); break;                                                                                \
+        case 6: CALL(6); break;                                                                                \
+        case 7: CALL(7); break;                                                                                \
+        case 8: CALL(8); break;                                                                                \
+        case 9: CALL(9); break;                                                                                \
+        case 10: CALL(10); break;                                                                              \
+        case 12: CALL(12); break;                                                                              \
+        case 15: CALL(15); break;                                                                              \
+        case 16: CALL(16); break;                                                                              \
+        default: CALL(0); break;                                                                               \
+    }
+
+// the multiply's radices: three components in registers
+#define MC_SWITCH_MUL(rad, CALL)                                                                               \
+    switch (rad) {                                                                                             \
+        case 1: CALL(1); break;                                                                                \
+        case 2: CALL(2); break;                                                                                \
+        case 3: CALL(3); break;                                                                                \
+        case 4: CALL(4); break;                                                                                \
+        case 5: CALL(5); break;                                                                                \
+        case 6: CALL(6); break;                                                                                \
+        case 7: CALL(7); break;                                                                                \
+        case 8: CALL(8); break;                                                                                \
+        default: CALL(0); break;                                                                               \
+    }
+
+// ---- forward stage 0: rows n < n_in of column `col` of component c (global) into the lines
+// (c, parity p), at (c*np + p)*N*TC.
+template <int R>
+__device__ __forceinline__ void first_fwd(const ColPlan& P, int rad, float2* sm, const float2* base,
+                                          long long comp_stride, long long ls, int n_in, int nh, int comps, int np, const float2* __restrict__ tw) {
+    const int TC = 1 << P.sh;
+    const int M = P.N / rad, per = M * TC;
+    for (int i = threadIdx.x; i < comps * per; i += blockDim.x) {
+        const int c = comps == 1 ? 0 : i / per, e = i - c * per;
+        const int col = e & (TC - 1), j = e >> P.sh;
+        const float2* g = base + c * comp_stride + col;
+        float2 x[RegLen<R>::n];
+        MC_EACH(r, rad) {
+            const int n = j + r * M;
+            x[r] = (col < nh && n < n_in) ? g[n * ls] : make_float2(0.f, 0.f);
+        }
+        for (int p = 0; p < np; p++) {
+            float2 v[RegLen<R>::n];
+            MC_EACH(r, rad) v[r] = p ? cmul(x[r], tw_l<-1>(P, tw, j + r * M)) : x[r];
+            dft_r<R, -1>(v, rad, P, tw);
+            float2* dst = sm + ((c * np + p) * P.N + j) * TC + col;
+            MC_EACH(k, rad) dst[k * M * TC] = j * k == 0 ? v[k] : cmul(v[k], tw_l<-1>(P, tw, j * k * P.NP));
+        }
+    }
+}
+
+// ---- a middle stage of sub-blocks of ncur elements (forward, or its mirror image)
+template <int R, int SIGN>
+__device__ __forceinline__ void mid_stage(const ColPlan& P, int rad, int ncur, float2* sm, int lines,
+                                          const float2* __restrict__ tw) {
+    const int TC = 1 << P.sh;
+    const int M = ncur / rad, per = P.N / rad * TC, ts = P.N / ncur * P.NP;
+    for (int i = threadIdx.x; i < lines * per; i += blockDim.x) {
+        const int l = i / per, e = i - l * per;
+        const int col = e & (TC - 1), q = e >> P.sh;
+        const int blk = q / M, j = q - blk * M;
+        float2* x = sm + (l * P.N + blk * ncur + j) * TC + col;
+        float2 v[RegLen<R>::n];
+        MC_EACH(r, rad) {
+            v[r] = x[r * M * TC];
+            if (SIGN > 0 && j * r) v[r] = cmul(v[r], tw_l<+1>(P, tw, j * r * ts));
+        }
+        dft_r<R, SIGN>(v, rad, P, tw);
+        MC_EACH(k, rad) x[k * M * TC] = (SIGN < 0 && j * k) ? cmul(v[k], tw_l<-1>(P, tw, j * k * ts)) : v[k];
+    }
+}
+
+// frequency of slot q of the last stage's sub-block: digits of q, most significant = stage 0
+__device__ __forceinline__ int slot_freq(const ColPlan& P, int q) {
+    if (P.nst <= 2) return q;
+    int f = 0, rest = P.nq, base = 1;
+    for (int s = 0; s < P.nst - 1; s++) {
+        rest /= P.r[s];
+        const int d = q / rest;
+        q -= d * rest;
+        f += d * base;
+        base *= P.r[s];
+    }
+    return f;
+}
+
+// ---- last forward stage to global rows (row NP*k + parity, rows < n_out)
+template <int R>
+__device__ __forceinline__ void last_fwd(const ColPlan& P, int rad, const float2* sm, float2* base, long long ls,
+                                         int n_out, int nh, int p0, const float2* __restrict__ tw) {
+    const int TC = 1 << P.sh;
+    for (int i = threadIdx.x; i < P.nq * TC; i += blockDim.x) {
+        const int col = i & (TC - 1), q = i >> P.sh;
+        float2 v[RegLen<R>::n];
+        MC_EACH(r, rad) v[r] = sm[(q * rad + r) * TC + col];
+        dft_r<R, -1>(v, rad, P, tw);
+        const int f = slot_freq(P, q);
+        if (col >= nh) continue;
+        MC_EACH(k, rad) {
+            const int row = P.NP * (f + k * P.nq) + p0;
+            if (row < n_out) base[row * ls + col] = v[k];
+        }
+    }
+}
+
+// ---- first inverse stage from global rows (< n_in) into the np parity lines
+template <int R>
+__device__ __forceinline__ void first_inv(const ColPlan& P, int rad, float2* sm, const float2* base, long long ls,
+                                          int n_in, int nh, const float2* __restrict__ tw) {
+    const int TC = 1 << P.sh;
+    const int per = P.nq * TC;
+    for (int i = threadIdx.x; i < P.NP * per; i += blockDim.x) {
+        const int p = P.NP == 1 ? 0 : i / per, e = i - p * per;
+        const int col = e & (TC - 1), q = e >> P.sh;
+        const int f = slot_freq(P, q);
+        float2 v[RegLen<R>::n];
+        MC_EACH(k, rad) {
+            const int row = P.NP * (f + k * P.nq) + p;
+            v[k] = (col < nh && row < n_in) ? base[row * ls + col] : make_float2(0.f, 0.f);
+        }
+        dft_r<R, +1>(v, rad, P, tw);
+        MC_EACH(r, rad) sm[(p * P.N + q * rad + r) * TC + col] = v[r];
+    }
+}
+
+// ---- last inverse stage: the parities' sum to global rows n < n_out
+template <int R>
+__device__ __forceinline__ void last_inv(const ColPlan& P, int rad, const float2* sm, float2* base,
+                                         long long comp_stride, long long ls, int n_out, int nh, int comps,
+                                         const float2* __restrict__ tw) {
+    const int TC = 1 << P.sh;
+    const int M = P.N / rad, per = M * TC;
+    for (int i = threadIdx.x; i < comps * per; i += blockDim.x) {
+        const int c = comps == 1 ? 0 : i / per, e = i - c * per;
+        const int col = e & (TC - 1), j = e >> P.sh;
+        float2 acc[RegLen<R>::n];
+        for (int p = 0; p < P.NP; p++) {
+            const float2* x = sm + ((c * P.NP + p) * P.N + j) * TC + col;
+            float2 v[RegLen<R>::n];
+            MC_EACH(k, rad) v[k] = j * k == 0 ? x[k * M * TC] : cmul(x[k * M * TC], tw_l<+1>(P, tw, j * k * P.NP));
+            dft_r<R, +1>(v, rad, P, tw);
+            MC_EACH(r, rad) acc[r] = p ? cadd(acc[r], cmul(v[r], tw_l<+1>(P, tw, j + r * M))) : v[r];
+        }
+        if (col >= nh) continue;
+        MC_EACH(r, rad) {
+            const int n = j + r * M;
+            if (n < n_out) base[c * comp_stride + n * ls + col] = acc[r];
+        }
+    }
+}
+
+// ---- last forward stage of the three components, H = K M, first inverse stage
+template <int R>
+__device__ __forceinline__ void mul_stage(const ColPlan& P, int rad, float2* sm, const KernelView& K, int kaxis, int o,
+                                          int kx0, int nh, float scale, const float2* __restrict__ tw) {
+    const int TC = 1 << P.sh;
+    const int per = P.nq * TC, cs = P.NP * P.N * TC;
+    for (int i = threadIdx.x; i < P.NP * per; i += blockDim.x) {
+        const int p = P.NP == 1 ? 0 : i / per, e = i - p * per;
+        const int col = e & (TC - 1), q = e >> P.sh;
+        if (col >= nh) continue;
+        float2* x = sm + (p * P.N + q * rad) * TC + col;
+        float2 a[RegLen<R>::n], b[RegLen<R>::n], c[RegLen<R>::n];
+        MC_EACH(r, rad) {
+            a[r] = x[r * TC];
+            b[r] = x[cs + r * TC];
+            c[r] = x[2 * cs + r * TC];
+        }
+        dft_r<R, -1>(a, rad, P, tw);
+        dft_r<R, -1>(b, rad, P, tw);
+        dft_r<R, -1>(c, rad, P, tw);
+        const int f = slot_freq(P, q);
+        MC_EACH(k, rad) {
+            const int fr = P.NP * (f + k * P.nq) + p;
+            float kk[6];
+            if (kaxis == 0) kernel_at(K, fr, o, kx0 + col, kk);
+            else kernel_at(K, 0, fr, kx0 + col, kk);
+            const float2 m0 = a[k], m1 = b[k], m2 = c[k];
+            // q: 0 xx, 1 yy, 2 zz, 3 yz, 4 xz, 5 xy
+            a[k] = make_float2(scale * (kk[0] * m0.x + kk[5] * m1.x + kk[4] * m2.x),
+                               scale * (kk[0] * m0.y + kk[5] * m1.y + kk[4] * m2.y));
+            b[k] = make_float2(scale * (kk[5] * m0.x + kk[1] * m1.x + kk[3] * m2.x),
+                               scale * (kk[5] * m0.y + kk[1] * m1.y + kk[3] * m2.y));
+            c[k] = make_float2(scale * (kk[4] * m0.x + kk[3] * m1.x + kk[2] * m2.x),
+                               scale * (kk[4] * m0.y + kk[3] * m1.y + kk[2] * m2.y));
+        }
+        dft_r<R, +1>(a, rad, P, tw);
+        dft_r<R, +1>(b, rad, P, tw);
+        dft_r<R, +1>(c, rad, P, tw);
+        MC_EACH(r, rad) {
+            x[r * TC] = a[r];
+            x[cs + r * TC] = b[r];
+            x[2 * cs + r * TC] = c[r];
+        }
+    }
+}
+
+template <int SIGN>
+__device__ __forceinline__ void mid_stages(const ColPlan& P, float2* sm, int lines, const float2* __restrict__ tw) {
+    if (SIGN < 0) {
+        int ncur = P.N / P.r[0];
+        for (int s = 1; s < P.nst - 1; s++) {
+#define CALL(R) mid_stage<R, -1>(P, P.r[s], ncur, sm, lines, tw)
+            MC_SWITCH(P.r[s], CALL)
+#undef CALL
+            ncur /= P.r[s];
+            __syncthreads();
+        }
+    } else {
+        int ncur = P.r[P.nst - 1];
+        for (int s = P.nst - 2; s > 0; s--) {
+            ncur *= P.r[s];
+#define CALL(R) mid_stage<R, +1>(P, P.r[s], ncur, sm, lines, tw)
+            MC_SWITCH(P.r[s], CALL)
+#undef CALL
+            __syncthreads();
+        }
+    }
+}
+
+// One component per line; block: outer index o, tile of TC columns.
+template <int SIGN>
+__global__ void __launch_bounds__(256, 2) colmix_fft_kernel(float2* __restrict__ S, int ncols, long long outer_stride,
+                                                         long long ls, int n_in, int n_out, ColPlan P,
+                                                         const float2* __restrict__ tw, const DevCtl* ctl,
+                                                         int skip_retry, long long sim_stride) {
+    pdl_begin();
+    if (ctl) ctl += blockIdx.y;
+    if (conv_skip(ctl, skip_retry)) return;
+    S += blockIdx.y * sim_stride;
+    const int TC = 1 << P.sh;
+    extern __shared__ unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    const int ntiles = (ncols + TC - 1) / TC;
+    const int o = blockIdx.x / ntiles;
+    const int kx0 = (blockIdx.x - o * ntiles) * TC;
+    const int nh = min(TC, ncols - kx0);
+    float2* base = S + (long long)o * outer_stride + kx0;
+    const int first = P.r[0], last = P.r[P.nst - 1];
+    if (SIGN < 0) {
+#define CALL(R) first_fwd<R>(P, first, sm, base, 0, ls, n_in, nh, 1, P.NP, tw)
+        MC_SWITCH(first, CALL)
+#undef CALL
+        __syncthreads();
+        mid_stages<-1>(P, sm, P.NP, tw);
+        for (int p = 0; p < P.NP; p++) {
+#define CALL(R) last_fwd<R>(P, last, sm + p * P.N * TC, base, ls, n_out, nh, p, tw)
+            MC_SWITCH(last, CALL)
+#undef CALL
+        }
+    } else {
+#define CALL(R) first_inv<R>(P, last, sm, base, ls, n_in, nh, tw)
+        MC_SWITCH(last, CALL)
+#undef CALL
+        __syncthreads();
+        mid_stages<+1>(P, sm, P.NP, tw);
+#define CALL(R) last_inv<R>(P, first, sm, base, 0, ls, n_out, nh, 1, tw)
+        MC_SWITCH(first, CALL)
+#undef CALL
+    }
+}
+
+// Three components per column: forward, symmetric kernel multiply, inverse.  kaxis 0: lines
+// along z (ky = o), 1: along y (kz = 0).
+__global__ void __launch_bounds__(256, 2) colmix_mul_kernel(float2* __restrict__ S, KernelView K, int ncols,
+                                                         long long comp_stride, long long outer_stride, long long ls,
+                                                         int n_in, int kaxis, float scale, ColPlan P,
+                                                         const float2* __restrict__ tw, const DevCtl* ctl,
+                                                         int skip_retry, long long sim_stride,
+                                                         const float* __restrict__ sim_scale) {
+    pdl_begin();
+    if (ctl) ctl += blockIdx.y;
+    if (conv_skip(ctl, skip_retry)) return;
+    S += blockIdx.y * sim_stride;
+    if (sim_scale) scale = sim_scale[blockIdx.y];
+    const int TC = 1 << P.sh;
+    extern __shared__ unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    const int ntiles = (ncols + TC - 1) / TC;
+    const int o = blockIdx.x / ntiles;
+    const int kx0 = (blockIdx.x - o * ntiles) * TC;
+    const int nh = min(TC, ncols - kx0);
+    float2* base = S + (long long)o * outer_stride + kx0;
+    const int first = P.r[0], last = P.r[P.nst - 1];
+#define CALL(R) first_fwd<R>(P, first, sm, base, comp_stride, ls, n_in, nh, 3, P.NP, tw)
+    MC_SWITCH(first, CALL)
+#undef CALL
+    __syncthreads();
+    mid_stages<-1>(P, sm, 3 * P.NP, tw);
+#define CALL(R) mul_stage<R>(P, last, sm, K, kaxis, o, kx0, nh, scale, tw)
+    MC_SWITCH_MUL(last, CALL)
+#undef CALL
+    __syncthreads();
+    mid_stages<+1>(P, sm, 3 * P.NP, tw);
+#define CALL(R) last_inv<R>(P, first, sm, base, comp_stride, ls, n_in, nh, 3, tw)
+    MC_SWITCH(first, CALL)
+#undef CALL
+}
+
+// The fewest stages of radices <= 16 (or one prime up to 31), then the smallest largest
+// radix, in descending order; at least two stages (a radix 1 after a prime length).
+bool radix_search(int n, int left, int most, int* out, int depth, int* best) {
+    if (left == 0) {
+        if (n != 1) return false;
+        for (int i = 0; i < depth; i++) best[i] = out[i];
+        return true;
+    }
+    for (int r = 2; r <= most; r++) {
+        const bool ok = r <= 10 || r == 12 || r == 15 || r == 16 || r == 11 || r == 13 || r == 17 || r == 19 || r == 23 || r == 29 || r == 31;
+        if (!ok || n % r) continue;
+        // descending: the first radix is the largest, so the smallest first choice wins
+        out[depth] = r;
+        if (radix_search(n / r, left - 1, r, out, depth + 1, best)) return true;
+    }
+    return false;
+}
+
+bool col_plan(int L, bool split, bool mul, const float2* tw_pow2, ColPlan* P, const float2** tw) {
+    P->NP = split ? 2 : 1;
+    P->N = L / P->NP;
+    int out[MC_MAXST], best[MC_MAXST] = {0};
+    P->nst = 0;
+    if (P->N == 1) {
+        best[0] = best[1] = 1;
+        P->nst = 2;
+    }
+    for (int k = 1; k < MC_MAXST && !P->nst; k++)
+        if (radix_search(P->N, k, 31, out, 0, best)) P->nst = k;
+    if (!P->nst) return false;
+    if (P->nst == 1) {
+        // a short composite length in two stages, a prime one with a trivial second stage
+        if (radix_search(P->N, 2, 31, out, 0, best)) P->nst = 2;
+        else best[P->nst++] = 1;
+    }
+    // the multiply keeps three components of the last radix in registers: at most 8, or a
+    // prime (a composite one always splits further)
+    auto prime = [](int r) { return r == 11 || r == 13 || r > 16; };
+    while (mul && best[P->nst - 1] > 8 && !prime(best[P->nst - 1])) {
+        if (!radix_search(P->N, P->nst + 1, 31, out, 0, best)) return false;
+        P->nst++;
+    }
+    for (int s = 0; s < P->nst; s++) P->r[s] = best[s];
+    P->nq = P->N / P->r[P->nst - 1];
+    if (mr_pow2(L)) {
+        P->tws = TWN / L;
+        *tw = tw_pow2;
+        return true;
+    }
+    P->tws = 1;
+    return mr_tables(L, tw, nullptr);
+}
+
+template <typename KT> cudaError_t mc_smem(KT kern, size_t bytes) {
+    if (bytes > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    return cudaSuccess;
+}
+
+// Columns per block: 16 (128-byte rows) while the lines fit 48 KB, fewer for longer lines
+// (2 at most 200 KB) and for grids of less than one block per SM.
+int pick_cols(size_t line_bytes, int ncols, long long outer) {
+    int tc = 16;
+    while (tc > 4 && line_bytes * tc > 50 * 1024) tc /= 2;
+    while (tc > 2 && line_bytes * tc > 200 * 1024) tc /= 2;
+    while (tc > 4 && (ncols + tc - 1) / tc * outer < 148) tc /= 2;
+    return tc;
+}
+
+int pick_threads(int work) { return std::min(256, std::max(64, (work + 31) / 32 * 32)); }
+
+}  // namespace
+
+cudaError_t launch_colmix_fft(int L, int sign, float2* S, int ncols, int nouter, long long outer_stride,
+                              long long line_stride, int n_in, int n_out, const float2* tw_pow2, const DevCtl* ctl,
+                              int skip_retry, cudaStream_t st, int nsim, long long sim_stride) {
+    ColPlan P;
+    const float2* tw = nullptr;
+    if (!col_plan(L, L % 2 == 0 && 2 * std::min(n_in, n_out) <= L, false, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
+    const size_t line = (size_t)P.NP * P.N * sizeof(float2);
+    const int tc = pick_cols(line, ncols, (long long)nouter * nsim);
+    const size_t smem = line * tc;
+    P.sh = tc == 16 ? 4 : (tc == 8 ? 3 : (tc == 4 ? 2 : 1));
+    const int threads = pick_threads(P.NP * P.nq * tc);
+    const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
+    cudaError_t e;
+    auto kern = sign < 0 ? colmix_fft_kernel<-1> : colmix_fft_kernel<1>;
+    if ((e = mc_smem(kern, smem)) != cudaSuccess) return e;
+    return launch_pdl(kern, grid, dim3(threads), smem, st, S, ncols, outer_stride, line_stride, n_in, n_out, P, tw, ctl,
+                      skip_retry, sim_stride);
+}
+
+cudaError_t launch_colmix_mul(int L, float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
+                              long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
+                              const float2* tw_pow2, const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+                              long long sim_stride, const float* sim_scale, int tile) {
+    ColPlan P;
+    const float2* tw = nullptr;
+    if (!col_plan(L, L % 2 == 0 && 2 * n_in <= L, true, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
+    const size_t line = (size_t)3 * P.NP * P.N * sizeof(float2);
+    int tc = pick_cols(line, ncols, (long long)nouter * nsim);
+    if (tile < 0 && tc > 2) tc /= 2;
+    if (tile > 0 && tc < 16 && line * tc * 2 <= 200 * 1024) tc *= 2;
+    const size_t smem = line * tc;
+    P.sh = tc == 16 ? 4 : (tc == 8 ? 3 : (tc == 4 ? 2 : 1));
+    if (smem > 220 * 1024) return cudaErrorNotSupported;
+    const int threads = pick_threads(std::max(P.NP * P.nq, 3 * P.N / P.r[0]) * tc);
+    const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
+    cudaError_t e;
+    if ((e = mc_smem(colmix_mul_kernel, smem)) != cudaSuccess) return e;
+    return launch_pdl(colmix_mul_kernel, grid, dim3(threads), smem, st, S, K, ncols, comp_stride, outer_stride,
+                      line_stride, n_in, kaxis, scale, P, tw, ctl, skip_retry, sim_stride, sim_scale);
+}
+
+}  // namespace mm

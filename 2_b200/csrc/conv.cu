@@ -219,63 +219,6 @@ __global__ void colfft_kernel(V* __restrict__ S, int ncols, long long outer_stri
     tile_store<L, TC, V>(sm, base, line_stride, n_out, nh, 0);
 }
 
-// ---------------------------------------------------------------- multiply pass
-// Three components per column: forward transform, H_d = sum_s Khat_sd M_s (symmetric,
-// real), inverse transform.  kaxis = 0: the line runs along z (ky = outer index);
-// kaxis = 1: the line runs along y (kz = 0, 2-D films).
-template <int L>
-__global__ void colmul_kernel(float2* __restrict__ S, KernelView K, int ncols, long long comp_stride,
-                              long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
-                              const float2* __restrict__ tw, const DevCtl* ctl, int skip_retry, long long sim_stride,
-                              const float* __restrict__ sim_scale) {
-    if (ctl) ctl += blockIdx.y;
-    if (conv_skip(ctl, skip_retry)) return;
-    S += blockIdx.y * sim_stride;
-    if (sim_scale) scale = sim_scale[blockIdx.y];
-    constexpr int TC = col_tile(L, 3, 8);
-    constexpr int TPL = tpl(L);
-    constexpr int LL = line_len(L);
-    extern __shared__ unsigned char smem_raw[];
-    float2* sm = reinterpret_cast<float2*>(smem_raw);
-    const int ntiles = (ncols + TC - 1) / TC;
-    const int o = blockIdx.x / ntiles;
-    const int kx0 = (blockIdx.x % ntiles) * TC;
-    const int nh = min(TC, ncols - kx0);
-    float2* base = S + (long long)o * outer_stride + kx0;
-#pragma unroll 1
-    for (int c = 0; c < 3; c++) tile_load<L, TC, float2>(sm, base + c * comp_stride, line_stride, n_in, nh, c * TC, true);
-    __syncthreads();
-    const int col = threadIdx.x / TPL;
-    const int t = threadIdx.x % TPL;
-    const bool act = col < TC;
-#pragma unroll 1
-    for (int c = 0; c < 3; c++) fft_line<L, -1, float2>(sm + (c * TC + (act ? col : 0)) * LL, t, act, tw);
-    for (int i = threadIdx.x; i < L * TC; i += blockDim.x) {
-        const int e = i / TC, c2 = i % TC;
-        const int kx = kx0 + c2;
-        if (c2 >= nh) continue;
-        float kk[6];
-        if (kaxis == 0) kernel_at(K, e, o, kx, kk);
-        else kernel_at(K, 0, e, kx, kk);
-        const int p = padx(e);
-        float2 m0 = sm[(0 * TC + c2) * LL + p];
-        float2 m1 = sm[(1 * TC + c2) * LL + p];
-        float2 m2 = sm[(2 * TC + c2) * LL + p];
-        // q: 0 xx, 1 yy, 2 zz, 3 yz, 4 xz, 5 xy
-        sm[(0 * TC + c2) * LL + p] = make_float2(scale * (kk[0] * m0.x + kk[5] * m1.x + kk[4] * m2.x),
-                                                 scale * (kk[0] * m0.y + kk[5] * m1.y + kk[4] * m2.y));
-        sm[(1 * TC + c2) * LL + p] = make_float2(scale * (kk[5] * m0.x + kk[1] * m1.x + kk[3] * m2.x),
-                                                 scale * (kk[5] * m0.y + kk[1] * m1.y + kk[3] * m2.y));
-        sm[(2 * TC + c2) * LL + p] = make_float2(scale * (kk[4] * m0.x + kk[3] * m1.x + kk[2] * m2.x),
-                                                 scale * (kk[4] * m0.y + kk[3] * m1.y + kk[2] * m2.y));
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int c = 0; c < 3; c++) fft_line<L, +1, float2>(sm + (c * TC + (act ? col : 0)) * LL, t, act, tw);
-#pragma unroll 1
-    for (int c = 0; c < 3; c++) tile_store<L, TC, float2>(sm, base + c * comp_stride, line_stride, n_in, nh, c * TC);
-}
-
 // ---------------------------------------------------------------- register z-multiply
 // The 3-D z pass without shared memory.  With the z direction zero-padded to
 // L0 = 2P (P = N0 non-zero planes), the forward transform splits into its even and odd
@@ -868,7 +811,10 @@ cudaError_t launch_colfft(int L, int sign, V* S, int ncols, int nouter, long lon
             }
         }
     }
-    if (sign < 0) {
+    if constexpr (sizeof(V) == 8) {
+        return launch_colmix_fft(L, sign, S, ncols, nouter, outer_stride, line_stride, n_in, n_out, tw, ctl,
+                                 skip_retry, st, nsim, sim_stride);
+    } else if (sign < 0) {
         switch (L) {
 #define X(l) case l: return launch_colfft_t<l, -1, V>(S, ncols, nouter, outer_stride, line_stride, n_in, n_out, tw, ctl, skip_retry, st, nsim, sim_stride);
             MM_FOR_POW2(X)
@@ -887,24 +833,6 @@ cudaError_t launch_colfft(int L, int sign, V* S, int ncols, int nouter, long lon
                                            skip_retry, st, nsim, sim_stride);
         }
     }
-}
-
-template <int L>
-static cudaError_t launch_colmul_t(float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
-                                   long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
-                                   const float2* tw, const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
-                                   long long sim_stride, const float* sim_scale) {
-    constexpr int TC = col_tile(L, 3, 8);
-    const size_t smem = (size_t)3 * TC * line_len(L) * sizeof(float2);
-    cudaError_t e = set_smem(colmul_kernel<L>, smem);
-    if (e != cudaSuccess) return e;
-    int ntiles = (ncols + TC - 1) / TC;
-    int threads = TC * tpl(L);
-    if (threads < 32) threads = 32;
-    colmul_kernel<L><<<dim3((unsigned)(nouter * ntiles), (unsigned)nsim), threads, smem, st>>>(
-        S, K, ncols, comp_stride, outer_stride, line_stride, n_in, kaxis, scale, tw, ctl, skip_retry, sim_stride,
-        sim_scale);
-    return cudaGetLastError();
 }
 
 // columns per block: 64 / P2 (192 threads) by default, halved or doubled by the tile
@@ -953,7 +881,8 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
                           const float2* tw, const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
                           long long sim_stride, const float* sim_scale, int tile) {
     if (kaxis == 1 && nouter == 1 && L >= 4 && L <= 1024) {
-        // single-layer films: the four-step column pass
+        // single-layer films: the four-step column pass (128x128 disk, RK45 step 148 us; with
+        // the in-place columns of colmix.cu 210 us)
         switch (L) {
 #define X(l) case l: return launch_colmul4_t<l>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, nsim, sim_stride, sim_scale, tile);
             X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024)
@@ -961,14 +890,8 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
             default: break;
         }
     }
-    switch (L) {
-#define X(l) case l: return launch_colmul_t<l>(S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, kaxis, scale, tw, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
-        MM_FOR_POW2(X)
-#undef X
-        default:
-            return launch_mr_colmul(L, S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, kaxis, scale,
-                                    ctl, skip_retry, st, nsim, sim_stride, sim_scale);
-    }
+    return launch_colmix_mul(L, S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, kaxis, scale, tw,
+                             ctl, skip_retry, st, nsim, sim_stride, sim_scale, tile);
 }
 
 template cudaError_t launch_xfwd<float2, float>(int, const float*, PP, const float*, float2*, int, int, int, int, int,

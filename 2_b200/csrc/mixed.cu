@@ -256,92 +256,12 @@ cudaError_t launch_mr_colfft(int L, int sign, V* S, int ncols, int nouter, long 
     return cudaGetLastError();
 }
 
-// Three components per column: forward transforms, H = sum_s K_sd M_s (symmetric, real
-// kernel from the stored octant), inverse transforms; kaxis 0: lines along z (ky = outer
-// index), kaxis 1: lines along y (kz = 0, single-layer films).  The three components are
-// transformed one after the other through one scratch line per column.
-__global__ void __launch_bounds__(256) mr_colmul_kernel(float2* __restrict__ S, KernelView K, int ncols,
-                                                        long long comp_stride, long long outer_stride,
-                                                        long long line_stride, int n_in, int kaxis, float scale,
-                                                        MrLine f, const float2* __restrict__ tw, const DevCtl* ctl,
-                                                        int skip_retry, long long sim_stride,
-                                                        const float* __restrict__ sim_scale, int TC) {
-    if (ctl) ctl += blockIdx.y;
-    if (conv_skip(ctl, skip_retry)) return;
-    S += blockIdx.y * sim_stride;
-    if (sim_scale) scale = sim_scale[blockIdx.y];
-    const int L = f.L;
-    extern __shared__ unsigned char smem_raw[];
-    float2* sm = reinterpret_cast<float2*>(smem_raw);  // [3][TC][L] lines, then [TC][L] scratch
-    const int ntiles = (ncols + TC - 1) / TC;
-    const int o = blockIdx.x / ntiles;
-    const int kx0 = (blockIdx.x % ntiles) * TC;
-    const int nh = min(TC, ncols - kx0);
-    float2* base = S + (long long)o * outer_stride + kx0;
-    for (int c = 0; c < 3; c++)
-        for (int i = threadIdx.x; i < L * TC; i += blockDim.x) {
-            const int e = i / TC, col = i % TC;
-            sm[(c * TC + col) * L + e] =
-                (e < n_in && col < nh) ? base[c * comp_stride + e * line_stride + col] : make_float2(0.f, 0.f);
-        }
-    const int nt = blockDim.x / TC;
-    const int col = threadIdx.x / nt, t = threadIdx.x % nt;
-    const bool act = col < TC;
-    const int cc = act ? col : 0;
-    float2* scratch = sm + (3 * TC + cc) * L;
-    for (int c = 0; c < 3; c++) mr_fft<-1, float2>(sm + (c * TC + cc) * L, scratch, f, tw, t, nt, act);
-    for (int i = threadIdx.x; i < L * TC; i += blockDim.x) {
-        const int e = i / TC, c2 = i % TC;
-        if (c2 >= nh) continue;
-        const int kx = kx0 + c2;
-        float kk[6];
-        if (kaxis == 0) kernel_at(K, e, o, kx, kk);
-        else kernel_at(K, 0, e, kx, kk);
-        const float2 m0 = sm[(0 * TC + c2) * L + e];
-        const float2 m1 = sm[(1 * TC + c2) * L + e];
-        const float2 m2 = sm[(2 * TC + c2) * L + e];
-        // q: 0 xx, 1 yy, 2 zz, 3 yz, 4 xz, 5 xy
-        sm[(0 * TC + c2) * L + e] = make_float2(scale * (kk[0] * m0.x + kk[5] * m1.x + kk[4] * m2.x),
-                                                scale * (kk[0] * m0.y + kk[5] * m1.y + kk[4] * m2.y));
-        sm[(1 * TC + c2) * L + e] = make_float2(scale * (kk[5] * m0.x + kk[1] * m1.x + kk[3] * m2.x),
-                                                scale * (kk[5] * m0.y + kk[1] * m1.y + kk[3] * m2.y));
-        sm[(2 * TC + c2) * L + e] = make_float2(scale * (kk[4] * m0.x + kk[3] * m1.x + kk[2] * m2.x),
-                                                scale * (kk[4] * m0.y + kk[3] * m1.y + kk[2] * m2.y));
-    }
-    for (int c = 0; c < 3; c++) mr_fft<+1, float2>(sm + (c * TC + cc) * L, scratch, f, tw, t, nt, act);
-    for (int c = 0; c < 3; c++)
-        for (int i = threadIdx.x; i < n_in * TC; i += blockDim.x) {
-            const int e = i / TC, c2 = i % TC;
-            if (c2 < nh) base[c * comp_stride + e * line_stride + c2] = sm[(c * TC + c2) * L + e];
-        }
-}
-
-cudaError_t launch_mr_colmul(int L, float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
-                             long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
-                             const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim, long long sim_stride,
-                             const float* sim_scale) {
-    MrLine f;
-    const float2* tw = nullptr;
-    if (!mr_factor(L, &f) || !table_of<float2>(L, &tw)) return cudaErrorInvalidValue;
-    const int TC = mr_cols(L, 4, sizeof(float2));
-    const size_t smem = (size_t)4 * TC * L * sizeof(float2);
-    cudaError_t e = mr_smem(mr_colmul_kernel, smem);
-    if (e != cudaSuccess) return e;
-    const int ntiles = (ncols + TC - 1) / TC;
-    mr_colmul_kernel<<<dim3((unsigned)(nouter * ntiles), (unsigned)nsim), 256, smem, st>>>(
-        S, K, ncols, comp_stride, outer_stride, line_stride, n_in, kaxis, scale, f, tw, ctl, skip_retry, sim_stride,
-        sim_scale, TC);
-    return cudaGetLastError();
-}
-
 template cudaError_t launch_mr_xfwd<float2, float>(int, const float*, PP, const float*, float2*, int, int, int, int,
                                                    int, int, int, const DevCtl*, int, cudaStream_t, int, long long,
                                                    long long, long long);
 template cudaError_t launch_mr_xfwd<double2, double>(int, const double*, PP, const float*, double2*, int, int, int,
                                                      int, int, int, int, const DevCtl*, int, cudaStream_t, int,
                                                      long long, long long, long long);
-template cudaError_t launch_mr_colfft<float2>(int, int, float2*, int, int, long long, long long, int, int,
-                                              const DevCtl*, int, cudaStream_t, int, long long);
 template cudaError_t launch_mr_colfft<double2>(int, int, double2*, int, int, long long, long long, int, int,
                                                const DevCtl*, int, cudaStream_t, int, long long);
 

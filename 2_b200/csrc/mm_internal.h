@@ -285,10 +285,15 @@ template <typename V>
 cudaError_t launch_mr_colfft(int L, int sign, V* S, int ncols, int nouter, long long outer_stride,
                              long long line_stride, int n_in, int n_out, const DevCtl* ctl, int skip_retry,
                              cudaStream_t st, int nsim, long long sim_stride);
-cudaError_t launch_mr_colmul(int L, float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
-                             long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
-                             const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim, long long sim_stride,
-                             const float* sim_scale);
+// column passes of any length (colmix.cu); lengths that are not powers of two need their
+// table prepared.  `tile` halves or doubles the columns per block of the multiply.
+cudaError_t launch_colmix_fft(int L, int sign, float2* S, int ncols, int nouter, long long outer_stride,
+                              long long line_stride, int n_in, int n_out, const float2* tw_pow2, const DevCtl* ctl,
+                              int skip_retry, cudaStream_t st, int nsim, long long sim_stride);
+cudaError_t launch_colmix_mul(int L, float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
+                              long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
+                              const float2* tw_pow2, const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+                              long long sim_stride, const float* sim_scale, int tile);
 // whether the C2R + epilogue pass for row length M can also write the R2C rows of the
 // next stage state (EpiArgs::fwd)
 bool epi_r2c_supported(int M);
