@@ -17,91 +17,15 @@
 // the last one writes it: a 3x3 multiply of two-stage columns needs two barriers.
 #include <algorithm>
 
+#include "colmix.cuh"
 #include "kernel_view.cuh"
-#include "mixed.cuh"
 #include "mm_internal.h"
 #include "pdl.cuh"
-#include "rdft.cuh"
 
 namespace mm {
 using namespace mmfft;
 
-constexpr int MC_MAXST = 12;
-
-struct ColPlan {
-    int N, NP, nst;
-    int r[MC_MAXST];  // radices in the order of the forward stages; the last one is the smallest
-    int nq;           // N / r[nst - 1]
-    int tws;          // W_L^m = tw[m * tws]
-    int sh;           // log2 of the columns per block (TC)
-};
-
 namespace {
-
-// a run-time radix 17..31 (prime): the paired sums of dft_prime on a local array, constants
-// from the twiddle table (W_R^m = tw[m * step])
-template <int SIGN>
-__device__ __noinline__ void dft_any(float2* a, int R, const float2* __restrict__ tw, int step) {
-    const int H = (R - 1) / 2;
-    float2 s[16], d[16];
-    float2 sum = a[0];
-    for (int n = 1; n <= H; n++) {
-        s[n] = cadd(a[n], a[R - n]);
-        d[n] = csub(a[n], a[R - n]);
-        sum = cadd(sum, s[n]);
-    }
-    const float2 a0 = a[0];
-    a[0] = sum;
-    for (int k = 1; k <= H; k++) {
-        float2 A = a0, B = make_float2(0.f, 0.f);
-        int m = 0;
-        for (int n = 1; n <= H; n++) {
-            m += k;
-            if (m >= R) m -= R;
-            const float2 w = tw[m * step];  // cos, -sin
-            A.x += w.x * s[n].x;
-            A.y += w.x * s[n].y;
-            B.x -= w.y * d[n].x;
-            B.y -= w.y * d[n].y;
-        }
-        const float2 iB = mul_si<SIGN>(B);
-        a[k] = cadd(A, iB);
-        a[R - k] = csub(A, iB);
-    }
-}
-
-// R = 0: the run-time radix `rad`
-template <int R, int SIGN>
-__device__ __forceinline__ void dft_r(float2* v, int rad, const ColPlan& P, const float2* __restrict__ tw) {
-    if constexpr (R > 0) RDft<R, SIGN>::run(v);
-    else dft_any<SIGN>(v, rad, tw, P.NP * P.N / rad * P.tws);
-}
-template <int R> struct RegLen { static constexpr int n = R > 0 ? R : 31; };
-
-template <int SIGN>
-__device__ __forceinline__ float2 tw_l(const ColPlan& P, const float2* __restrict__ tw, int m) {
-    const float2 w = __ldg(tw + m * P.tws);
-    return SIGN > 0 ? make_float2(w.x, -w.y) : w;
-}
-
-#define MC_EACH(r, rad) _Pragma("unroll") for (int r = 0; r < (R > 0 ? R : rad); r++)
-#define MC_SWITCH(rad, CALL)                                                                                   \
-    switch (rad) {                                                                                             \
-        case 1: CALL(1); break;                                                                                \
-        case 2: CALL(2); break;                                                                                \
-        case 3: CALL(3); break;                                                                                \
-        case 4: CALL(4); break;                                                                                \
-        case 5: CALL(5); break;                                                                                \
-        case 6: CALL(6); break;                                                                                \
-        case 7: CALL(7); break;                                                                                \
-        case 8: CALL(8); break;                                                                                \
-        case 9: CALL(9); break;                                                                                \
-        case 10: CALL(10); break;                                                                              \
-        case 12: CALL(12); break;                                                                              \
-        case 15: CALL(15); break;                                                                              \
-        case 16: CALL(16); break;                                                                              \
-        default: CALL(0); break;                                                                               \
-    }
 
 // the multiply's radices: three components in registers
 #define MC_SWITCH_MUL(rad, CALL)                                                                               \
@@ -141,41 +65,6 @@ __device__ __forceinline__ void first_fwd(const ColPlan& P, int rad, float2* sm,
             MC_EACH(k, rad) dst[k * M * TC] = j * k == 0 ? v[k] : cmul(v[k], tw_l<-1>(P, tw, j * k * P.NP));
         }
     }
-}
-
-// ---- a middle stage of sub-blocks of ncur elements (forward, or its mirror image)
-template <int R, int SIGN>
-__device__ __forceinline__ void mid_stage(const ColPlan& P, int rad, int ncur, float2* sm, int lines,
-                                          const float2* __restrict__ tw) {
-    const int TC = 1 << P.sh;
-    const int M = ncur / rad, per = P.N / rad * TC, ts = P.N / ncur * P.NP;
-    for (int i = threadIdx.x; i < lines * per; i += blockDim.x) {
-        const int l = i / per, e = i - l * per;
-        const int col = e & (TC - 1), q = e >> P.sh;
-        const int blk = q / M, j = q - blk * M;
-        float2* x = sm + (l * P.N + blk * ncur + j) * TC + col;
-        float2 v[RegLen<R>::n];
-        MC_EACH(r, rad) {
-            v[r] = x[r * M * TC];
-            if (SIGN > 0 && j * r) v[r] = cmul(v[r], tw_l<+1>(P, tw, j * r * ts));
-        }
-        dft_r<R, SIGN>(v, rad, P, tw);
-        MC_EACH(k, rad) x[k * M * TC] = (SIGN < 0 && j * k) ? cmul(v[k], tw_l<-1>(P, tw, j * k * ts)) : v[k];
-    }
-}
-
-// frequency of slot q of the last stage's sub-block: digits of q, most significant = stage 0
-__device__ __forceinline__ int slot_freq(const ColPlan& P, int q) {
-    if (P.nst <= 2) return q;
-    int f = 0, rest = P.nq, base = 1;
-    for (int s = 0; s < P.nst - 1; s++) {
-        rest /= P.r[s];
-        const int d = q / rest;
-        q -= d * rest;
-        f += d * base;
-        base *= P.r[s];
-    }
-    return f;
 }
 
 // ---- last forward stage to global rows (row NP*k + parity, rows < n_out)
@@ -315,7 +204,7 @@ __device__ __forceinline__ void mid_stages(const ColPlan& P, float2* sm, int lin
 // One component per line; block: outer index o, tile of TC columns.
 template <int SIGN>
 __global__ void __launch_bounds__(256, 2) colmix_fft_kernel(float2* __restrict__ S, int ncols, long long outer_stride,
-                                                         long long ls, int n_in, int n_out, ColPlan P,
+                                                         long long ls, int n_in, int n_out, const __grid_constant__ ColPlan P,
                                                          const float2* __restrict__ tw, const DevCtl* ctl,
                                                          int skip_retry, long long sim_stride) {
     pdl_begin();
@@ -358,7 +247,7 @@ __global__ void __launch_bounds__(256, 2) colmix_fft_kernel(float2* __restrict__
 // along z (ky = o), 1: along y (kz = 0).
 __global__ void __launch_bounds__(256, 2) colmix_mul_kernel(float2* __restrict__ S, KernelView K, int ncols,
                                                          long long comp_stride, long long outer_stride, long long ls,
-                                                         int n_in, int kaxis, float scale, ColPlan P,
+                                                         int n_in, int kaxis, float scale, const __grid_constant__ ColPlan P,
                                                          const float2* __restrict__ tw, const DevCtl* ctl,
                                                          int skip_retry, long long sim_stride,
                                                          const float* __restrict__ sim_scale) {
@@ -391,57 +280,22 @@ __global__ void __launch_bounds__(256, 2) colmix_mul_kernel(float2* __restrict__
 #undef CALL
 }
 
-// The fewest stages of radices <= 16 (or one prime up to 31), then the smallest largest
-// radix, in descending order; at least two stages (a radix 1 after a prime length).
-bool radix_search(int n, int left, int most, int* out, int depth, int* best) {
+bool mc_prime(int r) { return r == 11 || r == 13 || r > 16; }
+
+// `left` radices in descending order with product n, the smallest possible first one
+bool radix_search(int n, int left, int most, int cap, int* out, int depth, int* best) {
     if (left == 0) {
         if (n != 1) return false;
         for (int i = 0; i < depth; i++) best[i] = out[i];
         return true;
     }
     for (int r = 2; r <= most; r++) {
-        const bool ok = r <= 10 || r == 12 || r == 15 || r == 16 || r == 11 || r == 13 || r == 17 || r == 19 || r == 23 || r == 29 || r == 31;
+        const bool ok = (r <= cap && r != 14) || r == 11 || r == 13 || r == 17 || r == 19 || r == 23 || r == 29 || r == 31;
         if (!ok || n % r) continue;
-        // descending: the first radix is the largest, so the smallest first choice wins
         out[depth] = r;
-        if (radix_search(n / r, left - 1, r, out, depth + 1, best)) return true;
+        if (radix_search(n / r, left - 1, r, cap, out, depth + 1, best)) return true;
     }
     return false;
-}
-
-bool col_plan(int L, bool split, bool mul, const float2* tw_pow2, ColPlan* P, const float2** tw) {
-    P->NP = split ? 2 : 1;
-    P->N = L / P->NP;
-    int out[MC_MAXST], best[MC_MAXST] = {0};
-    P->nst = 0;
-    if (P->N == 1) {
-        best[0] = best[1] = 1;
-        P->nst = 2;
-    }
-    for (int k = 1; k < MC_MAXST && !P->nst; k++)
-        if (radix_search(P->N, k, 31, out, 0, best)) P->nst = k;
-    if (!P->nst) return false;
-    if (P->nst == 1) {
-        // a short composite length in two stages, a prime one with a trivial second stage
-        if (radix_search(P->N, 2, 31, out, 0, best)) P->nst = 2;
-        else best[P->nst++] = 1;
-    }
-    // the multiply keeps three components of the last radix in registers: at most 8, or a
-    // prime (a composite one always splits further)
-    auto prime = [](int r) { return r == 11 || r == 13 || r > 16; };
-    while (mul && best[P->nst - 1] > 8 && !prime(best[P->nst - 1])) {
-        if (!radix_search(P->N, P->nst + 1, 31, out, 0, best)) return false;
-        P->nst++;
-    }
-    for (int s = 0; s < P->nst; s++) P->r[s] = best[s];
-    P->nq = P->N / P->r[P->nst - 1];
-    if (mr_pow2(L)) {
-        P->tws = TWN / L;
-        *tw = tw_pow2;
-        return true;
-    }
-    P->tws = 1;
-    return mr_tables(L, tw, nullptr);
 }
 
 template <typename KT> cudaError_t mc_smem(KT kern, size_t bytes) {
@@ -463,16 +317,53 @@ int pick_threads(int work) { return std::min(256, std::max(64, (work + 31) / 32 
 
 }  // namespace
 
+// The fewest stages, then the smallest largest radix; at least two stages (a short composite
+// length in two, a prime one with a trivial second stage).
+bool col_plan(int L, bool split, int cap, int cap_last, const float2* tw_pow2, ColPlan* P, const float2** tw) {
+    P->NP = split ? 2 : 1;
+    P->N = L / P->NP;
+    int out[MC_MAXST], best[MC_MAXST] = {0};
+    P->nst = 0;
+    if (P->N == 1) {
+        best[0] = best[1] = 1;
+        P->nst = 2;
+    }
+    for (int k = 1; k < MC_MAXST && !P->nst; k++)
+        if (radix_search(P->N, k, 31, cap, out, 0, best)) P->nst = k;
+    if (!P->nst) return false;
+    if (P->nst == 1) {
+        if (radix_search(P->N, 2, 31, cap, out, 0, best)) P->nst = 2;
+        else best[P->nst++] = 1;
+    }
+    // a composite last radix always splits further
+    while (best[P->nst - 1] > cap_last && !mc_prime(best[P->nst - 1])) {
+        if (!radix_search(P->N, P->nst + 1, 31, cap, out, 0, best)) return false;
+        P->nst++;
+    }
+    for (int s = 0; s < P->nst; s++) P->r[s] = best[s];
+    P->nq = P->N / P->r[P->nst - 1];
+    P->sh = 0;
+    P->pitch = 1;
+    if (mr_pow2(L)) {
+        P->tws = TWN / L;
+        *tw = tw_pow2;
+        return true;
+    }
+    P->tws = 1;
+    return mr_tables(L, tw, nullptr);
+}
+
 cudaError_t launch_colmix_fft(int L, int sign, float2* S, int ncols, int nouter, long long outer_stride,
                               long long line_stride, int n_in, int n_out, const float2* tw_pow2, const DevCtl* ctl,
                               int skip_retry, cudaStream_t st, int nsim, long long sim_stride) {
     ColPlan P;
     const float2* tw = nullptr;
-    if (!col_plan(L, L % 2 == 0 && 2 * std::min(n_in, n_out) <= L, false, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
+    if (!col_plan(L, L % 2 == 0 && 2 * std::min(n_in, n_out) <= L, 16, 16, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
     const size_t line = (size_t)P.NP * P.N * sizeof(float2);
     const int tc = pick_cols(line, ncols, (long long)nouter * nsim);
     const size_t smem = line * tc;
     P.sh = tc == 16 ? 4 : (tc == 8 ? 3 : (tc == 4 ? 2 : 1));
+    P.pitch = tc;
     const int threads = pick_threads(P.NP * P.nq * tc);
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
     cudaError_t e;
@@ -488,13 +379,14 @@ cudaError_t launch_colmix_mul(int L, float2* S, const KernelView& K, int ncols, 
                               long long sim_stride, const float* sim_scale, int tile) {
     ColPlan P;
     const float2* tw = nullptr;
-    if (!col_plan(L, L % 2 == 0 && 2 * n_in <= L, true, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
+    if (!col_plan(L, L % 2 == 0 && 2 * n_in <= L, 16, 8, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
     const size_t line = (size_t)3 * P.NP * P.N * sizeof(float2);
     int tc = pick_cols(line, ncols, (long long)nouter * nsim);
     if (tile < 0 && tc > 2) tc /= 2;
     if (tile > 0 && tc < 16 && line * tc * 2 <= 200 * 1024) tc *= 2;
     const size_t smem = line * tc;
     P.sh = tc == 16 ? 4 : (tc == 8 ? 3 : (tc == 4 ? 2 : 1));
+    P.pitch = tc;
     if (smem > 220 * 1024) return cudaErrorNotSupported;
     const int threads = pick_threads(std::max(P.NP * P.nq, 3 * P.N / P.r[0]) * tc);
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);

@@ -7,13 +7,14 @@
 // for padded sizes such as 2^n * {3, 5, 7} (engine/gridsize.go:16-33), which the
 // reference convolves through cuFFT (fftplanX.go:59-64).  The C2R + epilogue pass of
 // these lengths is in rhs.cu (mr_xinv_epi_kernel).
+#include <algorithm>
 #include <cmath>
 #include <mutex>
 #include <vector>
 
-#include "kernel_view.cuh"
-#include "mixed.cuh"
+#include "colmix.cuh"
 #include "mm_internal.h"
+#include "pdl.cuh"
 
 namespace mm {
 using namespace mmfft;
@@ -188,6 +189,76 @@ cudaError_t launch_mr_xfwd(int M, const S* in, PP pp, const float* mask, V* out,
     return cudaGetLastError();
 }
 
+// The FP32 row pass: TC rows per block side by side in shared memory (colmix.cuh), a warp per
+// row between global memory and the transposed lines (pitch TC + 1: consecutive elements of
+// a row fall on distinct banks).
+__global__ void __launch_bounds__(256, 3) mr_rows_kernel(const float* __restrict__ in_fixed, PP in_pp,
+                                                         const float* __restrict__ mask, float2* __restrict__ out,
+                                                         int nrows, int Z, int Y, int Yout, int in_pitch, int n_in,
+                                                         int hp, const __grid_constant__ ColPlan P,
+                                                         const float2* __restrict__ twM,
+                                                         const float2* __restrict__ tw2M, const DevCtl* ctl,
+                                                         int skip_retry, long long in_bstride, long long out_bstride,
+                                                         long long mask_bstride) {
+    pdl_begin();
+    const int sim = blockIdx.y;
+    if (ctl) ctl += sim;
+    if (conv_skip(ctl, skip_retry)) return;
+    const float* in = (in_fixed ? in_fixed : in_pp.get(ctl ? ctl->cur : 0)) + sim * in_bstride;
+    out += sim * out_bstride;
+    if (mask) mask += sim * mask_bstride;
+    const int M = P.N, TC = 1 << P.sh;
+    extern __shared__ unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    unsigned short* slot = reinterpret_cast<unsigned short*>(sm + M * P.pitch);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    fill_slots(P, slot);
+    for (int l = warp; l < TC; l += nw) {
+        const int row = blockIdx.x * TC + l;
+        const float* src = in + (long long)row * in_pitch;
+        const float* msk = mask ? mask + (long long)(row % (Z * Y)) * in_pitch : nullptr;
+        const int n = row < nrows ? n_in : 0;
+        for (int e = lane; e < M; e += 32) {
+            float2 v = make_float2(0.f, 0.f);
+            if (2 * e < n) v.x = src[2 * e] * (msk ? msk[2 * e] : 1.f);
+            if (2 * e + 1 < n) v.y = src[2 * e + 1] * (msk ? msk[2 * e + 1] : 1.f);
+            sm[e * P.pitch + l] = v;
+        }
+    }
+    __syncthreads();
+    lines_fft<-1>(P, sm, twM);
+    for (int l = warp; l < TC; l += nw) {
+        const int row = blockIdx.x * TC + l;
+        if (row >= nrows) break;
+        const int c = row / (Z * Y), zy = row - c * (Z * Y);
+        const int z = zy / Y, y = zy - z * Y;
+        r2c_line(P, sm + l, slot, tw2M, lane, out + ((long long)(c * Z + z) * Yout + y) * hp);
+    }
+}
+
+template <>
+cudaError_t launch_mr_xfwd<float2, float>(int M, const float* in, PP pp, const float* mask, float2* out, int nrows,
+                                          int Z, int Y, int Yout, int in_pitch, int n_in, int hp, const DevCtl* ctl,
+                                          int skip_retry, cudaStream_t st, int nsim, long long in_bstride,
+                                          long long out_bstride, long long mask_bstride) {
+    ColPlan P;
+    const float2 *twM = nullptr, *tw2M = nullptr;
+    if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !table_of<float2>(2 * M, &tw2M)) return cudaErrorInvalidValue;
+    // 16 rows per block, fewer for long rows and for grids of less than two blocks per SM
+    int sh = 4;
+    while (sh > 2 && (lines_smem(M, 1 << sh) > 56 * 1024 || (long long)(nrows >> sh) * nsim < 296)) sh--;
+    while (sh > 0 && lines_smem(M, 1 << sh) > 200 * 1024) sh--;
+    P.sh = sh;
+    P.pitch = (1 << sh) + 1;
+    const size_t smem = lines_smem(M, 1 << sh);
+    cudaError_t e = mr_smem(mr_rows_kernel, smem);
+    if (e != cudaSuccess) return e;
+    const int tc = 1 << sh, threads = std::min(256, std::max(64, (tc * P.nq + 31) / 32 * 32));
+    return launch_pdl(mr_rows_kernel, dim3((unsigned)((nrows + tc - 1) / tc), (unsigned)nsim), dim3(threads), smem, st,
+                      in, pp, mask, out, nrows, Z, Y, Yout, in_pitch, n_in, hp, P, twM, tw2M, ctl, skip_retry,
+                      in_bstride, out_bstride, mask_bstride);
+}
+
 // ---------------------------------------------------------------- column passes
 // Columns per block: up to 16, as many as keep `lines` lines of L elements within 64 KB
 // (a single column may take up to 128 KB).
@@ -256,9 +327,6 @@ cudaError_t launch_mr_colfft(int L, int sign, V* S, int ncols, int nouter, long 
     return cudaGetLastError();
 }
 
-template cudaError_t launch_mr_xfwd<float2, float>(int, const float*, PP, const float*, float2*, int, int, int, int,
-                                                   int, int, int, const DevCtl*, int, cudaStream_t, int, long long,
-                                                   long long, long long);
 template cudaError_t launch_mr_xfwd<double2, double>(int, const double*, PP, const float*, double2*, int, int, int,
                                                      int, int, int, int, const DevCtl*, int, cudaStream_t, int,
                                                      long long, long long, long long);

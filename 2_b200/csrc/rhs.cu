@@ -18,7 +18,7 @@
 
 #include "fft.cuh"
 #include "fft4.cuh"
-#include "mixed.cuh"
+#include "colmix.cuh"
 #include "mm_internal.h"
 #include "kernel_view.cuh"
 #include "pdl.cuh"
@@ -565,9 +565,10 @@ __device__ __forceinline__ const SimScalars& pick_scalars(const SimScalars& stag
 // ---------------------------------------------------------------- C2R row pass + epilogue
 // Cells of the block's rows; H_demag of (row, c) at cell x is element x>>1 (real part for
 // even x, imaginary part for odd x) of shared-memory line (lrow*3 + c), stride LS.
+// TRANSP: the lines side by side, element e of line l at sm[e * LS + l].
 // FWD: float x of line (lrow, c) then takes the cell's next state (times the Msat mask
 // when A.fwd_mask) for the R2C rows of the next evaluation (four-step lines only).
-template <bool TERMS, bool PADDED, bool BATCH, bool FWD = false, int SPEC = 0>
+template <bool TERMS, bool PADDED, bool BATCH, bool FWD = false, int SPEC = 0, bool TRANSP = false>
 __device__ __forceinline__ void epilogue_rows(const EpiArgs& A, const SimScalars& S, const float2* sm, int LS,
                                               int row0, int nrow_here) {
     static_assert(!(FWD && (PADDED || TERMS)), "row output: four-step lines, no per-term outputs");
@@ -589,9 +590,10 @@ __device__ __forceinline__ void epilogue_rows(const EpiArgs& A, const SimScalars
     for (int e = threadIdx.x; e < total; e += blockDim.x) {
         const long long i = (long long)grow * n2 + x;
         const int pi = PADDED ? padx(x >> 1) : (x >> 1);
-        const float2 v0 = sm[(lrow * 3 + 0) * LS + pi];
-        const float2 v1 = sm[(lrow * 3 + 1) * LS + pi];
-        const float2 v2 = sm[(lrow * 3 + 2) * LS + pi];
+        const int at = TRANSP ? pi * LS + lrow * 3 : lrow * 3 * LS + pi, dc = TRANSP ? 1 : LS;
+        const float2 v0 = sm[at];
+        const float2 v1 = sm[at + dc];
+        const float2 v2 = sm[at + 2 * dc];
         const float3 hd = (x & 1) ? make_float3(v0.y, v1.y, v2.y) : make_float3(v0.x, v1.x, v2.x);
         if constexpr (FWD) {
             // float x of line (lrow, c) held H_demag of this cell only
@@ -1287,74 +1289,66 @@ static cudaError_t launch_xinv_t(const float2* S, int hp, int L1, const float2* 
 }
 
 // ---------------------------------------------------------------- mixed-radix C2R + epilogue
-// Row lengths M that are not powers of two: the pre-processing of xinv_epi_kernel, the
-// mixed-radix inverse transform of mixed.cuh, then the same epilogue.  rpb rows of three
-// component lines per block (line (row, c) at sm + (row*3 + c)*M, natural order; the
-// scratch lines follow), blockDim.x / (3 rpb) threads per line.  BATCH: the simulation's
-// scalars are staged in shared memory (batched plans, time tables).
+// Row lengths M that are not powers of two: rpb rows of three component lines side by side
+// in shared memory (colmix.cuh), a warp per spectrum row for the pre-processing, the in-place
+// inverse, then the same epilogue.  BATCH: the simulation's scalars are staged in shared
+// memory (batched plans, time tables).
 template <bool TERMS, bool BATCH, int SPEC>
-__global__ void __launch_bounds__(384) mr_xinv_epi_kernel(const float2* __restrict__ S, int hp, int L1, MrLine f,
+__global__ void __launch_bounds__(384, 2) mr_xinv_epi_kernel(const float2* __restrict__ S, int hp, int L1,
+                                                          const __grid_constant__ ColPlan P,
                                                           const float2* __restrict__ twM,
                                                           const float2* __restrict__ tw2M, EpiArgs A, int rpb) {
+    pdl_begin();
     const DevCtl* ctl = A.ctl ? A.ctl + blockIdx.y : nullptr;
     if (skip_eval(ctl, A.skip_retry)) return;
     S += blockIdx.y * A.spec_bstride;
-    {
-        const int nr = A.P.n[0] * A.P.n[1] - (int)blockIdx.x * rpb;
-        prefetch_epilogue_rows<BATCH>(A, (int)blockIdx.x * rpb, nr < rpb ? nr : rpb);
-    }
+    const int n0 = A.P.n[0], n1 = A.P.n[1];
+    const int row0 = (int)blockIdx.x * rpb;
+    const int here = min(rpb, n0 * n1 - row0);
+    prefetch_epilogue_rows<BATCH>(A, row0, here);
     __shared__ SimScalars s_sim;  // covered by the barriers of the transform
     if (BATCH && threadIdx.x == 0) stage_scalars(A, ctl, s_sim);
-    const int M = f.L;
-    const int nlines = 3 * rpb;
-    const int nt = blockDim.x / nlines;
-    const int li = threadIdx.x / nt, t = threadIdx.x % nt;
-    const int lr = li / 3, c = li % 3;
-    const int n0 = A.P.n[0], n1 = A.P.n[1];
-    const int nrows = n0 * n1;
-    const int row = blockIdx.x * rpb + lr;
-    const bool active = (li < nlines) && (row < nrows);
     extern __shared__ unsigned char smem_raw[];
     float2* sm = reinterpret_cast<float2*>(smem_raw);
-    const int lc = li < nlines ? li : 0;
-    float2* xl = sm + (size_t)lc * M;
-    float2* scratch = sm + (size_t)(nlines + lc) * M;
-    if (active) {
-        const int z = row / n1, y = row % n1;
-        const float2* src = S + ((long long)(c * n0 + z) * L1 + y) * hp;
-        // Z[k] = (X[k] + conj X[M-k]) + i W^-k (X[k] - conj X[M-k]),  W = exp(-2 pi i / 2M)
-        for (int k = t; k < M; k += nt) {
-            const float2 a = src[k], b = src[M - k];
-            const float2 s = make_float2(a.x + b.x, a.y - b.y);
-            const float2 d = make_float2(a.x - b.x, a.y + b.y);
-            const float2 w0 = tw2M[k];
-            const float2 wd = cmul(make_float2(w0.x, -w0.y), d);
-            xl[k] = make_float2(s.x - wd.y, s.y + wd.x);
-        }
+    unsigned short* slot = reinterpret_cast<unsigned short*>(sm + P.N * P.pitch);
+    fill_slots(P, slot);
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int l = warp; l < 3 * here; l += nw) {
+        const int row = row0 + l / 3, c = l % 3;
+        const int z = row / n1, y = row - z * n1;
+        c2r_line(P, sm + l, slot, tw2M, lane, S + ((long long)(c * n0 + z) * L1 + y) * hp);
     }
-    mr_fft<+1, float2>(xl, scratch, f, twM, t, nt, active);
-    const int row0 = blockIdx.x * rpb;
-    epilogue_rows<TERMS, false, BATCH, false, SPEC>(A, pick_scalars<BATCH>(s_sim, A.P.s), sm, M, row0,
-                                                    min(rpb, nrows - row0));
+    __syncthreads();
+    lines_fft<+1>(P, sm, twM);
+    epilogue_rows<TERMS, false, BATCH, false, SPEC, true>(A, pick_scalars<BATCH>(s_sim, A.P.s), sm, P.pitch, row0,
+                                                          here);
 }
 
-// rows per block and threads per line of the mixed-radix epilogue
-static void mr_xinv_shape(int M, int* rpb, int* nt) {
-    *nt = M >= 256 ? 128 : (M >= 64 ? 64 : 32);
-    *rpb = 384 / (3 * *nt) > 0 ? 384 / (3 * *nt) : 1;
-    while (*rpb > 1 && (size_t)*rpb * 6 * M * sizeof(float2) > 96 * 1024) *rpb /= 2;
+// Rows per block (5, 2 or 1: three lines each of 16, 8 or 4) and threads of the mixed-radix
+// epilogue: 16 lines while they fit 56 KB and leave two blocks per SM.
+static void mr_xinv_shape(int M, int n0n1, int n2, int nsim, int* rpb, int* sh, int* threads) {
+    *sh = 4;
+    *rpb = 5;
+    while (*sh > 2 && (lines_smem(M, 1 << *sh) > 56 * 1024 || (long long)((n0n1 + *rpb - 1) / *rpb) * nsim < 296)) {
+        (*sh)--;
+        *rpb = (1 << *sh) / 3;
+    }
+    const int cells = *rpb * n2, turns = (cells + 383) / 384;
+    *threads = std::max(96, ((cells + turns - 1) / turns + 31) / 32 * 32);
 }
 
 template <bool TERMS, bool BATCH>
 static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, const EpiArgs& A, cudaStream_t st,
                                     int* nblocks, int nsim) {
-    MrLine f;
+    ColPlan P;
     const float2 *twM = nullptr, *tw2M = nullptr;
-    if (!mr_factor(M, &f) || !mr_tables(M, &twM, nullptr) || !mr_tables(2 * M, &tw2M, nullptr))
+    if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !mr_tables(2 * M, &tw2M, nullptr))
         return cudaErrorInvalidValue;
-    int rpb, nt;
-    mr_xinv_shape(M, &rpb, &nt);
-    const size_t smem = (size_t)rpb * 6 * M * sizeof(float2);
+    int rpb, threads;
+    mr_xinv_shape(M, A.P.n[0] * A.P.n[1], A.P.n[2], nsim, &rpb, &P.sh, &threads);
+    P.pitch = (1 << P.sh) + 1;
+    const size_t smem = lines_smem(M, 1 << P.sh);
     // the epilogue without what the evaluation lacks (as the four-step pass chooses it)
     auto kern = mr_xinv_epi_kernel<TERMS, BATCH, 0>;
     if constexpr (!TERMS) {
@@ -1373,8 +1367,8 @@ static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, cons
     const int nrows = A.P.n[0] * A.P.n[1];
     const int blocks = (nrows + rpb - 1) / rpb;
     *nblocks = blocks;
-    kern<<<dim3((unsigned)blocks, (unsigned)nsim), 3 * rpb * nt, smem, st>>>(S, hp, L1, f, twM, tw2M, A, rpb);
-    return cudaGetLastError();
+    return launch_pdl(kern, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, S, hp, L1, P, twM, tw2M, A,
+                      rpb);
 }
 
 #endif  // MM_RHS_PART == 0
@@ -1486,12 +1480,7 @@ bool epi_r2c_supported(int M) { return use_xinv4(M); }
 // The most blocks per simulation that the pass may take for n0n1 rows (the size of the
 // reduction partials).
 int xinv_blocks(int M, int n0n1) {
-    if (!mr_pow2(M)) {
-        int rpb, nt;
-        mr_xinv_shape(M, &rpb, &nt);
-        return (n0n1 + rpb - 1) / rpb;
-    }
-    if (use_xinv4(M)) return n0n1;  // one row per block
+    if (!mr_pow2(M) || use_xinv4(M)) return n0n1;  // at least one row per block
     int TPL = mmfft::tpl(M);
     int rpb = (3 * TPL >= 384) ? 1 : 384 / (3 * TPL);
     size_t smem = (size_t)rpb * 3 * mmfft::line_len(M) * sizeof(float2);

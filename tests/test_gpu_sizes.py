@@ -1,6 +1,8 @@
 """The convolution passes at the sizes where their stages and tiles change: every length of
 the register z multiply, the in-place column transforms at one, two and three stages, prime,
-composite and power-of-two lengths, padded and periodic; demag field and torque against the FP64 oracle."""
+composite and power-of-two lengths, padded and periodic, and the row passes whose lengths are
+not powers of two; demag field and torque against the FP64 oracle."""
+import numpy as np
 import pytest
 
 from helpers import rand_m, rel_err, to_np
@@ -10,11 +12,12 @@ pytestmark = pytest.mark.gpu
 Z_LENGTHS = [(n0, 4, 6) for n0 in range(2, 18)]       # 2..16 in registers, 17 in columns
 COLUMNS = [(1, n1, 4) for n1 in (64, 65, 66, 75, 81, 96, 104, 128, 150, 169, 192, 217, 256, 300)]
 COLUMNS_3D = [(2, n1, 4) for n1 in (15, 17, 39, 48, 75, 121, 160, 200)] + [(32, 4, 4), (64, 3, 4), (36, 4, 4)]
+ROWS = [(1, 4, n2) for n2 in (3, 5, 7, 13, 15, 31, 75, 121, 150, 192, 250, 300, 341)] + [(2, 90, 12), (3, 25, 50)]
 
 
 # FP32 transforms of L points accumulate about eps * log2(L) <= 12 * 6e-8 relative to the
 # largest field: 1e-6 bounds them, with the kernel's own rounding
-@pytest.mark.parametrize("n", Z_LENGTHS + COLUMNS + COLUMNS_3D)
+@pytest.mark.parametrize("n", Z_LENGTHS + COLUMNS + COLUMNS_3D + ROWS)
 def test_demag_and_torque_at_size(n):
     import oracle as O
     from mumax2 import Plan
