@@ -13,6 +13,7 @@
 // kernel on the flipped, transposed weights.
 // conv3x3_wgrad: dW[co][tap][ci] = sum_p dY[p][co] X[p + tap][ci], M = co, N = (tap, ci),
 // K = pixels, split over blocks and accumulated in FP32 with atomics.
+#include <algorithm>
 #include <cuda_bf16.h>
 #include <cstdint>
 #include <cstdlib>
@@ -717,26 +718,29 @@ __device__ __forceinline__ bool mbar_wait(unsigned addr, unsigned parity, long l
 // band (two 8-channel planes, K-direction stride = plane size, 8-position groups 128
 // bytes apart) and the slice's weights for all nine taps; it is read from global memory
 // once instead of once per tap.  Pad positions are computed and not stored.
-constexpr int BAND_MAX = 128 + 2 * 257 + 2;  // widths up to 256
+__host__ __device__ constexpr int band_max(int T) { return 128 * T + 2 * 257 + 2; }  // widths up to 256
 
-template <int N, int ST>
+// A block computes T consecutive tiles of 128 positions, each in its own N TMEM columns, from
+// one band and one copy of the weights: the W+2 halo on both sides of the band (130 positions
+// beside 128 at W = 64) and the block's set-up are paid once per T tiles.
+template <int N, int ST, int T>
 __global__ void __launch_bounds__(256) conv3x3_tc_kernel(const bf16* __restrict__ in, int in_cs, int in_co, int Cin,
                                                          const bf16* __restrict__ W, const float* __restrict__ bias,
                                                          bf16* __restrict__ out, int out_cs, int out_co, int Cout,
                                                          int B, int H, int Wd, int relu, int* err, int band,
                                                          int stage_bytes, long long limit) {
     constexpr int M = 128;
-    constexpr int TCOLS = N < 32 ? 32 : N;         // TMEM columns (power of two >= 32)
+    constexpr int TCOLS = T * N < 32 ? 32 : T * N;  // TMEM columns (power of two >= 32)
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) unsigned long long mbar[ST];
     __shared__ unsigned tmem_base_sh;
     __shared__ int fail_sh;
-    __shared__ int s_q[BAND_MAX];                  // band position -> input pixel, or -1
+    __shared__ int s_q[band_max(T)];                  // band position -> input pixel, or -1
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int Wp = Wd + 1;
     const long long img = (long long)(H + 1) * Wp;
     const long long total = (long long)B * img;
-    const long long q0 = (long long)blockIdx.x * M;
+    const long long q0 = (long long)blockIdx.x * (M * T);
     const int n0 = blockIdx.y * N;
     const int plane = band * 16;                   // bytes of one 8-channel plane of the band
     const bool vec = (out_cs % 8 == 0) && (out_co % 8 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
@@ -807,13 +811,16 @@ __global__ void __launch_bounds__(256) conv3x3_tc_kernel(const bf16* __restrict_
 #pragma unroll 1
             for (int tap = 0; tap < 9; tap++) {
                 const unsigned off = (unsigned)(((tap / 3) * Wp + tap % 3) * 16);
-                const uint64_t ad = umma_desc(base + off, (unsigned)plane, 128);
                 const uint64_t bd = umma_desc(base + bwt + tap * N * 32, 128, 256);
                 const unsigned acc = (s > 0 || tap > 0) ? 1u : 0u;
-                asm volatile(
-                    "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                    " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem),
-                    "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+#pragma unroll
+                for (int t = 0; t < T; t++) {
+                    const uint64_t ad = umma_desc(base + off + t * M * 16, (unsigned)plane, 128);
+                    asm volatile(
+                        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                        " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(tmem + t * N),
+                        "l"(ad), "l"(bd), "r"(idesc), "r"(acc));
+                }
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(
                 smem_u32(&mbar[s % ST])));
@@ -844,26 +851,30 @@ __global__ void __launch_bounds__(256) conv3x3_tc_kernel(const bf16* __restrict_
     }
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (tile rows) and the column
-    // half w / 4 (N = 16: warps 0-3 take all columns); 16 columns per load
+    // epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 (tile rows) and the column half
+    // w / 4 of every tile (N = 16: all columns of every second tile); 16 columns per load
     constexpr int CW = N >= 32 ? N / 2 : N;
     const int quad = warp & 3, chalf = warp >> 2;
-    if (!fail_sh && chalf * CW < N) {
-        // this lane's output pixel (pad positions are not stored)
-        const int pix = s_q[quad * 32 + lane + Wp + 1];
+    if (!fail_sh) {
+        const int cb = CW < N ? chalf * CW : 0;
+#pragma unroll 1
+        for (int t = CW < N ? 0 : chalf; t < T; t += CW < N ? 1 : 2) {
+            // this lane's output pixel (pad positions are not stored)
+            const int pix = s_q[t * M + quad * 32 + lane + Wp + 1];
 #pragma unroll
-        for (int c0 = chalf * CW; c0 < chalf * CW + CW; c0 += 16) {
-            unsigned v[16];
-            const unsigned ta = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)c0;
-            asm volatile(
-                "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
-                "[%16];\n"
-                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                  "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
-                  "=r"(v[15])
-                : "r"(ta));
-            asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::);
-            if (pix >= 0) store16(v, out + (long long)pix * out_cs + out_co, n0 + c0, Cout, bias, relu, vec);
+            for (int c0 = cb; c0 < cb + CW; c0 += 16) {
+                unsigned v[16];
+                const unsigned ta = tmem + ((unsigned)(quad * 32) << 16) + (unsigned)(t * N + c0);
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, "
+                    "[%16];\n"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]),
+                      "=r"(v[15])
+                    : "r"(ta));
+                asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::);
+                if (pix >= 0) store16(v, out + (long long)pix * out_cs + out_co, n0 + c0, Cout, bias, relu, vec);
+            }
         }
     } else if (fail_sh && tid == 0) {
         atomicExch(err, 1);
@@ -876,36 +887,52 @@ __global__ void __launch_bounds__(256) conv3x3_tc_kernel(const bf16* __restrict_
     }
 }
 
-// Stages of the ring: as many (2..4) as fit in 110 KB, so that two blocks share an SM.
-template <int N, int ST>
+template <int N, int ST, int T>
 static cudaError_t launch_conv_tc_st(const bf16* in, int in_cs, int in_co, int Cin, const bf16* W, const float* bias,
                                      bf16* out, int out_cs, int out_co, int Cout, int B, int H, int Wd, int relu,
                                      int* err, cudaStream_t st, int band, int stage_bytes) {
     const int smem = ST * stage_bytes;
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_tc_kernel<N, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e =
+        cudaFuncSetAttribute(conv3x3_tc_kernel<N, ST, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const long long positions = (long long)B * (H + 1) * (Wd + 1);
-    dim3 grid((unsigned)((positions + 127) / 128), (unsigned)((Cout + N - 1) / N));
-    conv3x3_tc_kernel<N, ST><<<grid, 256, smem, st>>>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H,
-                                                      Wd, relu, err, band, stage_bytes, g_wait_limit);
+    dim3 grid((unsigned)((positions + 128 * T - 1) / (128 * T)), (unsigned)((Cout + N - 1) / N));
+    conv3x3_tc_kernel<N, ST, T><<<grid, 256, smem, st>>>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B,
+                                                         H, Wd, relu, err, band, stage_bytes, g_wait_limit);
     return cudaGetLastError();
 }
 
+// Stages of the ring: 2..4, one more than the layer has slices at most (a two-slice layer
+// keeps both in flight with three), and as many as fit in 110 KB, so that two blocks share an
+// SM.
+template <int N, int T>
+static cudaError_t launch_conv_tc_t(const bf16* in, int in_cs, int in_co, int Cin, const bf16* W, const float* bias,
+                                    bf16* out, int out_cs, int out_co, int Cout, int B, int H, int Wd, int relu,
+                                    int* err, cudaStream_t st) {
+    const int band = 128 * T + 2 * (Wd + 1) + 2;
+    const int stage_bytes = ((2 * band * 16 + 9 * N * 32) + 127) / 128 * 128;
+    const int fit = std::min((110 * 1024) / stage_bytes, Cin / 16 + 1);
+    if (fit >= 4)
+        return launch_conv_tc_st<N, 4, T>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu,
+                                          err, st, band, stage_bytes);
+    if (fit == 3)
+        return launch_conv_tc_st<N, 3, T>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu,
+                                          err, st, band, stage_bytes);
+    return launch_conv_tc_st<N, 2, T>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu, err,
+                                      st, band, stage_bytes);
+}
+
+// Tiles per block: 128 TMEM columns' worth (four for up to 32 output channels, two for 64; two
+// of 128 columns each for more), while that leaves two blocks per SM.
 template <int N>
 static cudaError_t launch_conv_tc(const bf16* in, int in_cs, int in_co, int Cin, const bf16* W, const float* bias,
                                   bf16* out, int out_cs, int out_co, int Cout, int B, int H, int Wd, int relu, int* err,
                                   cudaStream_t st) {
-    const int band = 128 + 2 * (Wd + 1) + 2;
-    const int stage_bytes = ((2 * band * 16 + 9 * N * 32) + 127) / 128 * 128;
-    const int fit = (110 * 1024) / stage_bytes;
-    if (fit >= 4)
-        return launch_conv_tc_st<N, 4>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu, err,
-                                       st, band, stage_bytes);
-    if (fit == 3)
-        return launch_conv_tc_st<N, 3>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu, err,
-                                       st, band, stage_bytes);
-    return launch_conv_tc_st<N, 2>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu, err, st,
-                                   band, stage_bytes);
+    constexpr int T = N <= 32 ? 4 : 2;
+    const long long blocks = ((long long)B * (H + 1) * (Wd + 1) / (128 * T)) * ((Cout + N - 1) / N);
+    if (blocks >= 2 * 148)
+        return launch_conv_tc_t<N, T>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu, err, st);
+    return launch_conv_tc_t<N, 1>(in, in_cs, in_co, Cin, W, bias, out, out_cs, out_co, Cout, B, H, Wd, relu, err, st);
 }
 
 // ---------------------------------------------------------------- tcgen05 convolution, persistent

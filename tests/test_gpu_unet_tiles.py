@@ -1,0 +1,39 @@
+"""The tcgen05 convolution with several position tiles per block, at the sizes where the
+tiles change; against float64 sums by torch of the same bf16 values."""
+import ctypes as C
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _p(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _taps(x, B, H, W, c):
+    """[9][B*H*W][c] float64: x at every tap, zero outside the image."""
+    import torch
+    xp = torch.nn.functional.pad(x.double().reshape(B, H, W, c), (0, 0, 1, 1, 1, 1))
+    return [xp[:, t // 3:t // 3 + H, t % 3:t % 3 + W].reshape(B * H * W, c) for t in range(9)]
+
+
+# enough positions for two blocks per SM of the widest tile; ragged widths; every tile of Cout
+@pytest.mark.parametrize("cin,cout,B,H,W", [(16, 16, 45, 64, 64), (32, 32, 40, 64, 64), (96, 32, 61, 41, 63),
+                                            (32, 48, 40, 40, 50), (64, 64, 20, 64, 64), (32, 96, 20, 64, 64),
+                                            (16, 136, 13, 64, 50), (32, 24, 1, 5, 3)])
+def test_conv_tiles(cin, cout, B, H, W):
+    import torch
+    from mumax2 import _native as nat
+    g = torch.Generator(device="cuda").manual_seed(cin + cout)
+    x = torch.randn(B * H * W, cin, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(cout, 9, cin, device="cuda", generator=g) / (9 * cin) ** 0.5).bfloat16()
+    b = torch.randn(cout, device="cuda", generator=g)
+    out = torch.zeros(B * H * W, cout, device="cuda", dtype=torch.bfloat16)
+    err = torch.zeros(1, device="cuda", dtype=torch.int32)
+    nat.check(nat.lib().mm_nn_conv3x3_tc(_p(x), cin, 0, cin, _p(w), _p(b), _p(out), cout, 0, cout, B, H, W, 0, _p(err),
+                                         None))
+    ref = b.double() + sum(v @ w[:, t].double().t() for t, v in enumerate(_taps(x, B, H, W, cin)))
+    assert int(err.item()) == 0
+    # one bf16 rounding (2^-9 of the value) and FP32 sums of up to 864 products
+    assert float(((out.double() - ref).abs() - 2.0 ** -8 * ref.abs()).max()) < 1e-4
