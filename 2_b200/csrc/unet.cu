@@ -261,6 +261,130 @@ __global__ void __launch_bounds__(128) conv3x3_wgrad_kernel(const bf16* __restri
         }
 }
 
+// The same sums with every input read once per tile.  A block owns 32 output x 32 input
+// channels for all nine taps and walks a range of the padded positions (band_pixel: a zero
+// column per row, a zero row per image, so border taps read zeros).  X runs through a ring of
+// positions in shared memory, [position][32 channels], in which the nine taps are row offsets;
+// a stage adds 64 positions of X and of dY, where the kernel above stages each tap's copy of
+// X, with its own index arithmetic, and 64 output channels whether the layer has them or not.
+// Six warps: three tap rows x two halves of the input channels; the 80-byte pitch keeps
+// ldmatrix free of bank conflicts.  Split over positions with FP32 reductions, two floats each
+// where dW is 8-byte aligned.
+constexpr int WR_KC = 64, WR_PITCH = 40, WR_THREADS = 192;
+
+__device__ __forceinline__ int band_pixel(int q, int total, int img, int Wp, int H, int Wd) {
+    if (q < 0 || q >= total) return -1;
+    const int b = q / img, r = q - b * img;
+    const int y = r / Wp, xp = r - y * Wp;
+    return (y < H && xp > 0) ? (b * H + y) * Wd + xp - 1 : -1;
+}
+
+__global__ void __launch_bounds__(WR_THREADS) conv3x3_wgrad_ring_kernel(
+    const bf16* __restrict__ dy, int dy_cs, int dy_co, int Cout, const bf16* __restrict__ x, int x_cs, int x_co,
+    int Cin, float* __restrict__ dW, int total, int img, int H, int Wd, int ring, int pos_per_block, int pairs) {
+    extern __shared__ __align__(128) unsigned char wr_smem[];
+    bf16* sB = reinterpret_cast<bf16*>(wr_smem);                    // [ring][WR_PITCH]
+    bf16* sA = sB + ring * WR_PITCH;                                // [2][WR_KC][WR_PITCH]
+    int* s_pix = reinterpret_cast<int*>(sA + 2 * WR_KC * WR_PITCH);  // [ring]
+    const int mask = ring - 1, Wp = Wd + 1;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int m0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
+    const int ps = blockIdx.z * pos_per_block;
+    const int pe = min(ps + pos_per_block, total);
+    auto pixels = [&](int q0, int n) {
+        for (int e = tid; e < n; e += WR_THREADS) s_pix[(q0 + e) & mask] = band_pixel(q0 + e, total, img, Wp, H, Wd);
+    };
+    auto load_x = [&](int q0, int n) {
+        for (int e = tid; e < 4 * n; e += WR_THREADS) {
+            const int slot = (q0 + (e >> 2)) & mask, ch = (e & 3) * 8, pix = s_pix[slot];
+            const bool ok = pix >= 0 && c0 + ch < Cin;
+            cp_async16(sB + slot * WR_PITCH + ch, x + (ok ? (long long)pix * x_cs + x_co + c0 + ch : 0), ok);
+        }
+    };
+    auto load_dy = [&](int st, int q0) {
+        for (int e = tid; e < 4 * WR_KC; e += WR_THREADS) {
+            const int row = e >> 2, ch = (e & 3) * 8, pix = s_pix[(q0 + row) & mask];
+            const bool ok = pix >= 0 && m0 + ch < Cout;
+            cp_async16(sA + (st * WR_KC + row) * WR_PITCH + ch,
+                       dy + (ok ? (long long)pix * dy_cs + dy_co + m0 + ch : 0), ok);
+        }
+    };
+    const int trow = warp % 3, half = (warp / 3) * 16;
+    const bool work = c0 + half < Cin;
+    float acc[2][3][2][4];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int t = 0; t < 3; t++)
+#pragma unroll
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int q = 0; q < 4; q++) acc[i][t][j][q] = 0.f;
+    // positions q - (Wp + 1) .. q + (Wp + 1) serve an output position q
+    pixels(ps - (Wp + 1), 2 * WR_KC + 2 * (Wp + 1));
+    __syncthreads();
+    load_x(ps - (Wp + 1), WR_KC + 2 * (Wp + 1));
+    load_dy(0, ps);
+    cp_commit();
+    int st = 0;
+    for (int q = ps; q < pe; q += WR_KC, st ^= 1) {
+        if (q + WR_KC < pe) {
+            load_x(q + WR_KC + Wp + 1, WR_KC);
+            load_dy(st ^ 1, q + WR_KC);
+            pixels(q + 2 * WR_KC + Wp + 1, WR_KC);
+        }
+        cp_commit();
+        cp_wait<1>();
+        __syncthreads();
+        if (work) {
+            const bf16* A = sA + st * WR_KC * WR_PITCH;
+#pragma unroll
+            for (int ks = 0; ks < WR_KC; ks += 16) {
+                unsigned a[2][4];
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    ldm_x4_t(a[i], A + (ks + (lane & 7) + ((lane >> 4) << 3)) * WR_PITCH + i * 16 +
+                                       ((lane >> 3) & 1) * 8);
+#pragma unroll
+                for (int t = 0; t < 3; t++) {
+                    unsigned b[4];
+                    const int slot = (q + ks + (trow - 1) * Wp + t - 1 + (lane & 15)) & mask;
+                    ldm_x4_t(b, sB + slot * WR_PITCH + half + (lane >> 4) * 8);
+#pragma unroll
+                    for (int i = 0; i < 2; i++)
+#pragma unroll
+                        for (int j = 0; j < 2; j++) mma_bf16(acc[i][t][j], a[i], b[2 * j], b[2 * j + 1]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (!work) return;
+    const int g = lane >> 2, t4 = lane & 3;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int hr = 0; hr < 2; hr++) {
+            const int co = m0 + i * 16 + g + hr * 8;
+            if (co >= Cout) continue;
+#pragma unroll
+            for (int t = 0; t < 3; t++)
+#pragma unroll
+                for (int j = 0; j < 2; j++) {
+                    const int ci = c0 + half + j * 8 + t4 * 2;
+                    if (ci >= Cin) continue;
+                    float* w = dW + ((long long)co * 9 + trow * 3 + t) * Cin + ci;
+                    const float v0 = acc[i][t][j][hr * 2], v1 = acc[i][t][j][hr * 2 + 1];
+                    if (pairs) {
+                        atomicAdd(reinterpret_cast<float2*>(w), make_float2(v0, v1));
+                    } else {
+                        atomicAdd(w, v0);
+                        atomicAdd(w + 1, v1);
+                    }
+                }
+        }
+}
+
 // ---------------------------------------------------------------- elementwise pieces
 // 2x2 average pool: out (H/2 x W/2) <- in (H x W), channel views
 // 2x2 average pooling, nearest upsampling and their gradients on NHWC views, 8 channels
@@ -530,6 +654,29 @@ extern "C" MM_API int mm_nn_conv3x3_wgrad(const void* dy, int dy_cs, int dy_co, 
         return report_error(MM_ERR_ARG, "mm_nn_conv3x3_wgrad: channel counts, strides and offsets must be multiples of 8");
     if ((long long)B * H * Wd >= (1LL << 30)) return report_error(MM_ERR_ARG, "mm_nn_conv3x3_wgrad: too many pixels");
     const long long P = (long long)B * H * Wd;
+    const long long total = (long long)B * (H + 1) * (Wd + 1);
+    int ring = 256;
+    while (ring < 3 * WR_KC + 2 * (Wd + 2)) ring *= 2;
+    // rows of up to 414 pixels (a ring of 1024 positions, two blocks per SM); longer ones
+    // keep the kernel that stages each tap
+    if (ring <= 1024 && total < (1LL << 30)) {
+        const size_t smem = (size_t)(ring + 2 * WR_KC) * WR_PITCH * sizeof(bf16) + (size_t)ring * sizeof(int);
+        const cudaError_t e = cudaFuncSetAttribute(conv3x3_wgrad_ring_kernel,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return report_error(MM_ERR_CUDA, cudaGetErrorString(e));
+        // three blocks per SM, at least four stages each (a block starts with 2 (W + 2)
+        // positions of halo and ends with 9216 reductions)
+        const int mt = (Cout + 31) / 32, nt = (Cin + 31) / 32;
+        const long long stages = (total + WR_KC - 1) / WR_KC;
+        long long per = (stages * mt * nt + 148 * 3 - 1) / (148 * 3);
+        per = std::min(stages, std::max(per, 4LL));
+        conv3x3_wgrad_ring_kernel<<<dim3((unsigned)mt, (unsigned)nt, (unsigned)((stages + per - 1) / per)), WR_THREADS,
+                                    smem, (cudaStream_t)st>>>(
+            (const bf16*)dy, dy_cs, dy_co, Cout, (const bf16*)x, x_cs, x_co, Cin, dW, (int)total, (H + 1) * (Wd + 1), H,
+            Wd, ring, (int)per * WR_KC, (reinterpret_cast<uintptr_t>(dW) & 7) == 0);
+        NN_CHECK();
+        return MM_OK;
+    }
     const int mt = (Cout + WG_BM - 1) / WG_BM, nt = (9 * Cin + WG_BN - 1) / WG_BN;
     // split the pixels so that about 4 waves of blocks cover the GPU
     long long splits = (148LL * 4 * 4 + mt * nt - 1) / (mt * nt);
@@ -1217,13 +1364,6 @@ static bool conv_persistent() {
 // ((dy+1)(W+1) + dx+1) positions, a 16-byte-aligned descriptor offset.  Blocks split
 // the positions; each adds its nine 128 x 32 partial sums to dW with FP32 atomics.
 constexpr int WGT_KC = 64;  // positions per stage
-
-__device__ __forceinline__ int band_pixel(int q, int total, int img, int Wp, int H, int Wd) {
-    if (q < 0 || q >= total) return -1;
-    const int b = q / img, r = q - b * img;
-    const int y = r / Wp, xp = r - y * Wp;
-    return (y < H && xp > 0) ? (b * H + y) * Wd + xp - 1 : -1;
-}
 
 constexpr int WGT_BAND_MAX = WGT_KC + 2 * 257 + 2;  // widths up to 256
 

@@ -1,5 +1,6 @@
-"""The tcgen05 convolution with several position tiles per block, at the sizes where the
-tiles change; against float64 sums by torch of the same bf16 values."""
+"""The tcgen05 convolution with several position tiles per block and the weight gradient's ring
+of positions, at the sizes where their tiles change; against float64 sums by torch of the same
+bf16 values."""
 import ctypes as C
 
 import pytest
@@ -37,3 +38,22 @@ def test_conv_tiles(cin, cout, B, H, W):
     assert int(err.item()) == 0
     # one bf16 rounding (2^-9 of the value) and FP32 sums of up to 864 products
     assert float(((out.double() - ref).abs() - 2.0 ** -8 * ref.abs()).max()) < 1e-4
+
+
+# a ring of 256, 512 and 1024 positions, rows too long for it, channel remainders, and a
+# gradient that is not 8-byte aligned
+@pytest.mark.parametrize("cin,cout,B,H,W,shift", [(16, 32, 1, 3, 5, 0), (32, 32, 70, 8, 8, 0), (24, 40, 3, 17, 33, 0),
+                                                  (96, 32, 2, 64, 64, 0), (64, 16, 2, 9, 200, 0), (8, 8, 1, 4, 413, 0),
+                                                  (16, 32, 1, 3, 450, 0), (32, 64, 2, 16, 16, 1)])
+def test_weight_gradient_ring(cin, cout, B, H, W, shift):
+    import torch
+    from mumax2 import _native as nat
+    g = torch.Generator(device="cuda").manual_seed(cin * cout + W)
+    x = torch.randn(B * H * W, cin, device="cuda", generator=g).bfloat16()
+    dy = torch.randn(B * H * W, cout, device="cuda", generator=g).bfloat16()
+    buf = torch.zeros(cout * 9 * cin + shift, device="cuda")
+    dw = buf[shift:]
+    nat.check(nat.lib().mm_nn_conv3x3_wgrad(_p(dy), cout, 0, cout, _p(x), cin, 0, cin, _p(dw), B, H, W, None))
+    ref = torch.stack([dy.double().t() @ v for v in _taps(x, B, H, W, cin)], 1).reshape(-1)
+    # FP32 sums of P products in a few hundred partial sums: eps * sqrt(P) of the norm and more
+    assert float((dw.double() - ref).norm() / ref.norm()) < 1e-5
