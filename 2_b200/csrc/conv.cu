@@ -17,6 +17,7 @@
 //
 // Column passes work on tiles of TC adjacent kx columns (TC a compile-time function
 // of the line length), so every global access moves TC*8 contiguous bytes.
+#include <algorithm>
 #include <cstdio>
 
 #include "fft.cuh"
@@ -835,12 +836,12 @@ cudaError_t launch_colfft(int L, int sign, V* S, int ncols, int nouter, long lon
     }
 }
 
-// columns per block: 64 / P2 (192 threads) by default, halved or doubled by the tile
+// columns per block: 64 / P2 (192 threads) by default, doubled or halved by the shift
 template <int L, int SHIFT>
 __host__ __device__ constexpr int colmul4_tc() {
-    constexpr int t0 = (64 / FS<L>::P2) > 0 ? 64 / FS<L>::P2 : 1;
-    constexpr int t = SHIFT > 0 ? t0 * 2 : (SHIFT < 0 ? t0 / 2 : t0);
-    return (t < 1 || t > 32 || 3 * t * FS<L>::P2 > 384) ? (t0 > 32 ? 32 : t0) : t;
+    constexpr int t0 = 64 / FS<L>::P2 > 32 ? 32 : 64 / FS<L>::P2;
+    constexpr int t = SHIFT > 0 ? t0 * 2 : t0 >> -SHIFT;
+    return t < 1 ? 1 : (t > 32 || 3 * t * FS<L>::P2 > 384) ? t0 : t;
 }
 
 template <int L, int SHIFT>
@@ -866,14 +867,22 @@ static cudaError_t launch_colmul4_t(float2* S, const KernelView& K, int ncols, l
                                     long long line_stride, int n_in, float scale, const float2* tw,
                                     const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
                                     long long sim_stride, const float* sim_scale, int tile) {
-    if (tile < 0)
-        return launch_colmul4_s<L, -1>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st,
-                                       nsim, sim_stride, sim_scale);
-    if (tile > 0)
-        return launch_colmul4_s<L, 1>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st,
-                                      nsim, sim_stride, sim_scale);
-    return launch_colmul4_s<L, 0>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, nsim,
-                                  sim_stride, sim_scale);
+    // single small films: fewer columns per block while the blocks leave SMs idle (a 128x32
+    // film has 129 columns, 17 blocks of the default 8)
+    int shift = tile;
+    const long long cols = (long long)ncols * nsim;
+    while (shift > -3 && cols < 148LL * (64 / FS<L>::P2 >> -std::min(shift, 0))) shift--;
+#define GO(sh)                                                                                                  \
+    return launch_colmul4_s<L, sh>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, \
+                                   nsim, sim_stride, sim_scale)
+    switch (shift) {
+        case 1: GO(1);
+        case 0: GO(0);
+        case -1: GO(-1);
+        case -2: GO(-2);
+        default: GO(-3);
+    }
+#undef GO
 }
 
 cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,

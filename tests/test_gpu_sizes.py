@@ -2,7 +2,6 @@
 the register z multiply, the in-place column transforms at one, two and three stages, prime,
 composite and power-of-two lengths, padded and periodic, and the row passes whose lengths are
 not powers of two; demag field and torque against the FP64 oracle."""
-import numpy as np
 import pytest
 
 from helpers import rand_m, rel_err, to_np
