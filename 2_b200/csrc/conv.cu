@@ -236,85 +236,101 @@ __device__ __forceinline__ float2 wtab(const float2* __restrict__ tw, int m, int
     return SIGN > 0 ? make_float2(w.x, -w.y) : w;
 }
 
+// BATCH: the block does `group` simulations one after the other with its columns' kernel
+// values in registers: they are the same for all, and with one simulation per block their 6 P
+// gathers per lane are twice the spectrum's 3 P loads.
 template <int P, bool BATCH>
 __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, KernelView K, int L1, int h, int hp,
                                                        long long comp_stride, long long zstride, float scale,
                                                        const float2* __restrict__ tw, int tws, const DevCtl* ctl,
                                                        int skip_retry, long long sim_stride,
-                                                       const float* __restrict__ sim_scale) {
+                                                       const float* __restrict__ sim_scale, int nsim, int group) {
     pdl_begin();
-    if (BATCH) {
-        if (ctl) ctl += blockIdx.y;
-        S += blockIdx.y * sim_stride;
-        if (sim_scale) scale = sim_scale[blockIdx.y];
-    }
-    if (conv_skip(ctl, skip_retry)) return;
+    if (!BATCH && conv_skip(ctl, skip_retry)) return;
     const long long gt = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     const int s = (int)(gt & 1);
     const long long colg = gt >> 1;
     const bool active = colg < (long long)L1 * h;
     const int ky = active ? (int)(colg / h) : 0;
     const int kx = active ? (int)(colg % h) : 0;
-    float2* base = S + (long long)ky * hp + kx;
-    float2 x[3][P];
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int z = 0; z < P; z++)
-            x[c][z] = active ? base[c * comp_stride + z * zstride] : make_float2(0.f, 0.f);
-    // odd outputs: pre-multiply by W_{2P}^z (forward)
-    if (s) {
-#pragma unroll
-        for (int z = 1; z < P; z++) {
-            const float2 w = wtab<-1>(tw, z, tws);
-#pragma unroll
-            for (int c = 0; c < 3; c++) x[c][z] = cmul(x[c][z], w);
-        }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; c++) RDft<P, -1>::run(x[c]);
-    // multiply: x[c][k'] holds X_c[kz], kz = 2k' + s
     const int kyy = (ky > (K.L1 >> 1)) ? K.L1 - ky : ky;
     const float sy = (ky > (K.L1 >> 1)) ? -1.f : 1.f;
     const int cs = K.kd0 * K.kd1 * K.kd2;
-#pragma unroll
-    for (int k = 0; k < P; k++) {
+    // the six kernel components at kz = 2k + s
+    auto kernel_of = [&](int k, float (&q)[6]) {
         int kz = 2 * k + s;
         float sz = 1.f;
         if (kz > P) { kz = 2 * P - kz; sz = -1.f; }
         const int idx = (kz * K.kd1 + kyy) * K.kd2 + kx;
-        const float kxx = __ldg(K.k + idx);
-        const float kyy_ = __ldg(K.k + cs + idx);
-        const float kzz = __ldg(K.k + 2 * cs + idx);
-        const float kyz = K.nz[3] ? sy * __ldg(K.k + 3 * cs + idx) : 0.f;
-        const float kxz = K.nz[4] ? sz * __ldg(K.k + 4 * cs + idx) : 0.f;
-        const float kxy = K.nz[5] ? sz * sy * __ldg(K.k + 5 * cs + idx) : 0.f;
-        const float2 m0 = x[0][k], m1 = x[1][k], m2 = x[2][k];
-        x[0][k] = make_float2(scale * (kxx * m0.x + kxy * m1.x + kxz * m2.x), scale * (kxx * m0.y + kxy * m1.y + kxz * m2.y));
-        x[1][k] = make_float2(scale * (kxy * m0.x + kyy_ * m1.x + kyz * m2.x), scale * (kxy * m0.y + kyy_ * m1.y + kyz * m2.y));
-        x[2][k] = make_float2(scale * (kxz * m0.x + kyz * m1.x + kzz * m2.x), scale * (kxz * m0.y + kyz * m1.y + kzz * m2.y));
+        q[0] = __ldg(K.k + idx);
+        q[1] = __ldg(K.k + cs + idx);
+        q[2] = __ldg(K.k + 2 * cs + idx);
+        q[3] = K.nz[3] ? sy * __ldg(K.k + 3 * cs + idx) : 0.f;
+        q[4] = K.nz[4] ? sz * __ldg(K.k + 4 * cs + idx) : 0.f;
+        q[5] = K.nz[5] ? sz * sy * __ldg(K.k + 5 * cs + idx) : 0.f;
+    };
+    constexpr bool KEEP = BATCH && P <= 8;  // longer columns leave no registers for them
+    float kv[KEEP ? P : 1][6];
+    if (KEEP) {
+#pragma unroll
+        for (int k = 0; k < P; k++) kernel_of(k, kv[KEEP ? k : 0]);
     }
+    const int sim0 = BATCH ? (int)blockIdx.y * group : 0, sim1 = BATCH ? min(sim0 + group, nsim) : 1;
+#pragma unroll 1
+    for (int sim = sim0; sim < sim1; sim++) {
+        if (BATCH && conv_skip(ctl ? ctl + sim : nullptr, skip_retry)) continue;
+        const float sc = BATCH && sim_scale ? sim_scale[sim] : scale;
+        float2* base = S + sim * sim_stride + (long long)ky * hp + kx;
+        float2 x[3][P];
 #pragma unroll
-    for (int c = 0; c < 3; c++) RDft<P, +1>::run(x[c]);
-    if (s) {
+        for (int c = 0; c < 3; c++)
 #pragma unroll
-        for (int z = 1; z < P; z++) {
-            const float2 w = wtab<+1>(tw, z, tws);
+            for (int z = 0; z < P; z++)
+                x[c][z] = active ? base[c * comp_stride + z * zstride] : make_float2(0.f, 0.f);
+        // odd outputs: pre-multiply by W_{2P}^z (forward)
+        if (s) {
 #pragma unroll
-            for (int c = 0; c < 3; c++) x[c][z] = cmul(x[c][z], w);
+            for (int z = 1; z < P; z++) {
+                const float2 w = wtab<-1>(tw, z, tws);
+#pragma unroll
+                for (int c = 0; c < 3; c++) x[c][z] = cmul(x[c][z], w);
+            }
         }
+#pragma unroll
+        for (int c = 0; c < 3; c++) RDft<P, -1>::run(x[c]);
+        // multiply: x[c][k'] holds X_c[kz], kz = 2k' + s; q: 0 xx, 1 yy, 2 zz, 3 yz, 4 xz, 5 xy
+#pragma unroll
+        for (int k = 0; k < P; k++) {
+            float kl[6];
+            if (!KEEP) kernel_of(k, kl);
+            const float(&q)[6] = KEEP ? kv[KEEP ? k : 0] : kl;
+            const float2 m0 = x[0][k], m1 = x[1][k], m2 = x[2][k];
+            x[0][k] = make_float2(sc * (q[0] * m0.x + q[5] * m1.x + q[4] * m2.x), sc * (q[0] * m0.y + q[5] * m1.y + q[4] * m2.y));
+            x[1][k] = make_float2(sc * (q[5] * m0.x + q[1] * m1.x + q[3] * m2.x), sc * (q[5] * m0.y + q[1] * m1.y + q[3] * m2.y));
+            x[2][k] = make_float2(sc * (q[4] * m0.x + q[3] * m1.x + q[2] * m2.x), sc * (q[4] * m0.y + q[3] * m1.y + q[2] * m2.y));
+        }
+#pragma unroll
+        for (int c = 0; c < 3; c++) RDft<P, +1>::run(x[c]);
+        if (s) {
+#pragma unroll
+            for (int z = 1; z < P; z++) {
+                const float2 w = wtab<+1>(tw, z, tws);
+#pragma unroll
+                for (int c = 0; c < 3; c++) x[c][z] = cmul(x[c][z], w);
+            }
+        }
+        // sum of the even and odd halves of the inverse; each lane stores half of the planes
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+#pragma unroll
+            for (int z = 0; z < P; z++) {
+                float2 v = x[c][z];
+                v.x += __shfl_xor_sync(0xffffffffu, v.x, 1);
+                v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
+                const bool mine = (z < (P + 1) / 2) == (s == 0);
+                if (active && mine) base[c * comp_stride + z * zstride] = v;
+            }
     }
-    // sum of the even and odd halves of the inverse; each lane stores half of the planes
-#pragma unroll
-    for (int c = 0; c < 3; c++)
-#pragma unroll
-        for (int z = 0; z < P; z++) {
-            float2 v = x[c][z];
-            v.x += __shfl_xor_sync(0xffffffffu, v.x, 1);
-            v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
-            const bool mine = (z < (P + 1) / 2) == (s == 0);
-            if (active && mine) base[c * comp_stride + z * zstride] = v;
-        }
 }
 
 // Four lanes per column (P >= 4): lane s computes the outputs kz = 4k' + s, k' < P/2,
@@ -432,12 +448,17 @@ static cudaError_t launch_zmul_reg_t(float2* S, const KernelView& K, int L1, int
                                      const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
                                      long long sim_stride, const float* sim_scale) {
     const long long threads = 2LL * L1 * h;
-    const dim3 grid((unsigned)((threads + 127) / 128), (unsigned)nsim);
-    if (nsim > 1)
-        return launch_pdl(zmul_reg_kernel<P, true>, grid, dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride,
-                          scale, tw, tws, ctl, skip_retry, sim_stride, sim_scale);
-    return launch_pdl(zmul_reg_kernel<P, false>, grid, dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride, scale,
-                      tw, tws, ctl, skip_retry, sim_stride, sim_scale);
+    const unsigned blocks = (unsigned)((threads + 127) / 128);
+    if (nsim > 1) {
+        // simulations per block: up to eight while 16 blocks per SM remain
+        int group = 8;
+        while (group > 1 && (long long)blocks * ((nsim + group - 1) / group) < 148 * 16) group /= 2;
+        return launch_pdl(zmul_reg_kernel<P, true>, dim3(blocks, (unsigned)((nsim + group - 1) / group)), dim3(128), 0,
+                          st, S, K, L1, h, hp, comp_stride, zstride, scale, tw, tws, ctl, skip_retry, sim_stride,
+                          sim_scale, nsim, group);
+    }
+    return launch_pdl(zmul_reg_kernel<P, false>, dim3(blocks), dim3(128), 0, st, S, K, L1, h, hp, comp_stride, zstride,
+                      scale, tw, tws, ctl, skip_retry, sim_stride, sim_scale, 1, 1);
 }
 
 template <int P>
