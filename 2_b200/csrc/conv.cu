@@ -639,13 +639,15 @@ __global__ void __launch_bounds__(512) xfwd4_kernel(const float* __restrict__ in
 // (3 x TC x P2 threads, rows n >= n_in are the zero padding and are not read), transformed,
 // put in natural order in shared memory, multiplied by the symmetric kernel there (all
 // three components of a (ky, kx) point meet in one thread), taken back into registers
-// and inverse-transformed; only the rows n < n_in are stored.  Replaces the Stockham
+// and inverse-transformed; only the rows n < n_in are stored.  ZAX: lines along z of bodies too
+// tall for the register multiply, one (ky, kx tile) per block.  Replaces the Stockham
 // colmul_kernel for 2-D films (seven barrier-separated stages per transform and
 // component there, two barriers per transform here).
-template <int L, int TC>
+template <int L, int TC, bool ZAX>
 __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, KernelView K, int ncols,
-                                                      long long comp_stride, long long line_stride, int n_in,
-                                                      float scale, const float2* __restrict__ tw, const DevCtl* ctl,
+                                                      long long comp_stride, long long outer_stride,
+                                                      long long line_stride, int n_in, float scale,
+                                                      const float2* __restrict__ tw, const DevCtl* ctl,
                                                       int skip_retry, long long sim_stride,
                                                       const float* __restrict__ sim_scale, int cstride) {
     pdl_begin();
@@ -659,12 +661,14 @@ __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, Ke
     const int per = TC * F::P2;                    // threads per component
     const int c = threadIdx.x / per, r = threadIdx.x - c * per;
     const int col = r % TC, t = r / TC;
-    const int kx0 = blockIdx.x * TC;
+    const int ntiles = (ncols + TC - 1) / TC;
+    const int o = ZAX ? (int)blockIdx.x / ntiles : 0;
+    const int kx0 = ((int)blockIdx.x - o * ntiles) * TC;
     const bool active = c < 3 && kx0 + col < ncols;
     float2* line = sm + ((c < 3 ? c : 0) * TC + col) * cstride;
     float2* twt = sm + 3 * TC * cstride;
     F::fill_twiddles(twt, tw);
-    float2* base = S + (long long)(c < 3 ? c : 0) * comp_stride + kx0 + col;
+    float2* base = S + (long long)(c < 3 ? c : 0) * comp_stride + o * outer_stride + kx0 + col;
     float2 v[F::P1];
 #pragma unroll
     for (int j = 0; j < F::P1; j++) {
@@ -684,7 +688,7 @@ __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, Ke
         const int ky = e / TC, c2 = e - ky * TC;
         if (c2 >= nh) continue;
         float kk[6];
-        kernel_at(K, 0, ky, kx0 + c2, kk);
+        kernel_at(K, ZAX ? ky : 0, ZAX ? o : ky, kx0 + c2, kk);
         float2* l0 = sm + (0 * TC + c2) * cstride + ky;
         float2* l1 = sm + (1 * TC + c2) * cstride + ky;
         float2* l2 = sm + (2 * TC + c2) * cstride + ky;
@@ -708,6 +712,86 @@ __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, Ke
     for (int q = 0; q < F::P1; q++) {
         const int n = F::out_index(t, q);
         if (active && n < n_in) base[n * line_stride] = v[q];
+    }
+}
+
+// The same for lines of 2H elements of which at most H are not padding, H too long for the
+// exchange buffers at 2H: by the parity of the frequency, X[2k] = DFT_H(x)[k] and
+// X[2k+1] = DFT_H(x W_2H^n)[k], one after the other; the inverse's first H rows are the sum of
+// the two inverses, the odd one times W_2H^-n, kept in registers.  The input is read twice (the
+// second time from L2) and written at the end.
+template <int H, int TC>
+__global__ void __launch_bounds__(3 * TC * FS<H>::P2, 1) colmul_split_kernel(
+    float2* __restrict__ S, KernelView K, int ncols, long long comp_stride, long long line_stride, int n_in, float scale,
+    const float2* __restrict__ tw, const DevCtl* ctl, int skip_retry, long long sim_stride,
+    const float* __restrict__ sim_scale, int cstride) {
+    pdl_begin();
+    if (ctl) ctl += blockIdx.y;
+    if (conv_skip(ctl, skip_retry)) return;
+    S += blockIdx.y * sim_stride;
+    if (sim_scale) scale = sim_scale[blockIdx.y];
+    using F = FS<H>;
+    extern __shared__ unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    constexpr int per = TC * F::P2;
+    const int c = threadIdx.x / per, r = threadIdx.x - c * per;
+    const int col = r % TC, t = r / TC;
+    const int kx0 = blockIdx.x * TC;
+    const bool active = kx0 + col < ncols;
+    float2* line = sm + (c * TC + col) * cstride;
+    float2* twt = sm + 3 * TC * cstride;
+    F::fill_twiddles(twt, tw);
+    float2* base = S + c * comp_stride + kx0 + col;
+    const int nh = min(TC, ncols - kx0);
+    float2 acc[F::P1];
+#pragma unroll 1
+    for (int p = 0; p < 2; p++) {
+        float2 v[F::P1];
+#pragma unroll
+        for (int j = 0; j < F::P1; j++) {
+            const int n = F::in_index(t, j);
+            v[j] = (active && n < n_in) ? base[n * line_stride] : make_float2(0.f, 0.f);
+            if (p) v[j] = cmul(v[j], TwSrc<-1, float2>::get(tw, n, 2 * H));
+        }
+        __syncthreads();
+        F::template run<-1>(v, line, t, active, twt, TC);
+        if (active) {
+#pragma unroll
+            for (int q = 0; q < F::P1; q++) line[F::out_index(t, q)] = v[q];
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < H * TC; e += blockDim.x) {
+            const int k = e / TC, c2 = e - k * TC;
+            if (c2 >= nh) continue;
+            float kk[6];
+            kernel_at(K, 0, 2 * k + p, kx0 + c2, kk);
+            float2* l0 = sm + (0 * TC + c2) * cstride + k;
+            float2* l1 = sm + (1 * TC + c2) * cstride + k;
+            float2* l2 = sm + (2 * TC + c2) * cstride + k;
+            const float2 m0 = *l0, m1 = *l1, m2 = *l2;
+            // q: 0 xx, 1 yy, 2 zz, 3 yz, 4 xz, 5 xy
+            *l0 = make_float2(scale * (kk[0] * m0.x + kk[5] * m1.x + kk[4] * m2.x),
+                              scale * (kk[0] * m0.y + kk[5] * m1.y + kk[4] * m2.y));
+            *l1 = make_float2(scale * (kk[5] * m0.x + kk[1] * m1.x + kk[3] * m2.x),
+                              scale * (kk[5] * m0.y + kk[1] * m1.y + kk[3] * m2.y));
+            *l2 = make_float2(scale * (kk[4] * m0.x + kk[3] * m1.x + kk[2] * m2.x),
+                              scale * (kk[4] * m0.y + kk[3] * m1.y + kk[2] * m2.y));
+        }
+        __syncthreads();
+        if (active) {
+#pragma unroll
+            for (int j = 0; j < F::P1; j++) v[j] = line[F::in_index(t, j)];
+        }
+        __syncthreads();
+        F::template run<+1>(v, line, t, active, twt, TC);
+#pragma unroll
+        for (int q = 0; q < F::P1; q++)
+            acc[q] = p ? cadd(acc[q], cmul(v[q], TwSrc<+1, float2>::get(tw, F::out_index(t, q), 2 * H))) : v[q];
+    }
+#pragma unroll
+    for (int q = 0; q < F::P1; q++) {
+        const int n = F::out_index(t, q);
+        if (active && n < n_in) base[n * line_stride] = acc[q];
     }
 }
 
@@ -865,22 +949,38 @@ __host__ __device__ constexpr int colmul4_tc() {
     return t < 1 ? 1 : (t > 32 || 3 * t * FS<L>::P2 > 384) ? t0 : t;
 }
 
-template <int L, int SHIFT>
-static cudaError_t launch_colmul4_s(float2* S, const KernelView& K, int ncols, long long comp_stride,
-                                    long long line_stride, int n_in, float scale, const float2* tw,
-                                    const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+template <int L, int SHIFT, bool ZAX>
+static cudaError_t launch_colmul4_s(float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
+                                    long long outer_stride, long long line_stride, int n_in, float scale,
+                                    const float2* tw, const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
                                     long long sim_stride, const float* sim_scale) {
     using F = FS<L>;
     constexpr int TC = colmul4_tc<L, SHIFT>();
     const int cstride = col4_stride<L>(TC < 16 ? TC : 16) > F::LBUF ? col4_stride<L>(TC < 16 ? TC : 16) : F::LBUF;
     const size_t smem = (size_t)(3 * TC * cstride + F::TWT) * sizeof(float2);
-    cudaError_t e = set_smem(colmul4_kernel<L, TC>, smem);
+    cudaError_t e = set_smem(colmul4_kernel<L, TC, ZAX>, smem);
     if (e != cudaSuccess) return e;
     int threads = 3 * TC * F::P2;
     if (threads < 32) threads = 32;
     const int ntiles = (ncols + TC - 1) / TC;
-    return launch_pdl(colmul4_kernel<L, TC>, dim3((unsigned)ntiles, (unsigned)nsim), dim3(threads), smem, st, S, K, ncols,
-                      comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, sim_stride, sim_scale, cstride);
+    return launch_pdl(colmul4_kernel<L, TC, ZAX>, dim3((unsigned)(nouter * ntiles), (unsigned)nsim), dim3(threads), smem,
+                      st, S, K, ncols, comp_stride, outer_stride, line_stride, n_in, scale, tw, ctl, skip_retry,
+                      sim_stride, sim_scale, cstride);
+}
+
+// lines of 2H elements, n_in <= H of them not padding
+template <int H, int TC>
+static cudaError_t launch_colmul_split(float2* S, const KernelView& K, int ncols, long long comp_stride,
+                                       long long line_stride, int n_in, float scale, const float2* tw,
+                                       const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+                                       long long sim_stride, const float* sim_scale) {
+    const int cstride = col4_stride<H>(TC);
+    const size_t smem = (size_t)(3 * TC * cstride + FS<H>::TWT) * sizeof(float2);
+    cudaError_t e = set_smem(colmul_split_kernel<H, TC>, smem);
+    if (e != cudaSuccess) return e;
+    return launch_pdl(colmul_split_kernel<H, TC>, dim3((unsigned)((ncols + TC - 1) / TC), (unsigned)nsim),
+                      dim3(3 * TC * FS<H>::P2), smem, st, S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl,
+                      skip_retry, sim_stride, sim_scale, cstride);
 }
 
 template <int L>
@@ -894,8 +994,8 @@ static cudaError_t launch_colmul4_t(float2* S, const KernelView& K, int ncols, l
     const long long cols = (long long)ncols * nsim;
     while (shift > -3 && cols < 148LL * (64 / FS<L>::P2 >> -std::min(shift, 0))) shift--;
 #define GO(sh)                                                                                                  \
-    return launch_colmul4_s<L, sh>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, \
-                                   nsim, sim_stride, sim_scale)
+    return launch_colmul4_s<L, sh, false>(S, K, ncols, 1, comp_stride, 0, line_stride, n_in, scale, tw, ctl,    \
+                                          skip_retry, st, nsim, sim_stride, sim_scale)
     switch (shift) {
         case 1: GO(1);
         case 0: GO(0);
@@ -920,6 +1020,18 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
             default: break;
         }
     }
+    if (kaxis == 0) {
+        // tall bodies: the four-step pass along z
+        switch (L) {
+#define X(l) case l: return launch_colmul4_s<l, 0, true>(S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
+            X(8) X(16) X(32) X(64) X(128) X(256) X(512)
+#undef X
+            default: break;
+        }
+    }
+    if (kaxis == 1 && nouter == 1 && L == 2048 && 2 * n_in <= L)
+        return launch_colmul_split<1024, 4>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st,
+                                            nsim, sim_stride, sim_scale);
     return launch_colmix_mul(L, S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, kaxis, scale, tw,
                              ctl, skip_retry, st, nsim, sim_stride, sim_scale, tile);
 }
