@@ -599,10 +599,10 @@ __device__ __forceinline__ void epilogue_rows(const EpiArgs& A, const SimScalars
             // float x of line (lrow, c) held H_demag of this cell only
             float3 nx = make_float3(0.f, 0.f, 0.f);
             process_cell<TERMS, SPEC>(A, S, m, r, dbg, i, mo, z, y, x, hd, ns, dtth, tr, &nx);
-            float* fl = reinterpret_cast<float*>(const_cast<float2*>(sm)) + 2 * (long long)(lrow * 3) * LS + x;
+            float* fl = reinterpret_cast<float*>(const_cast<float2*>(sm)) + 2 * at + (x & 1);
             fl[0] = nx.x;
-            fl[2 * LS] = nx.y;
-            fl[4 * LS] = nx.z;
+            fl[2 * dc] = nx.y;
+            fl[4 * dc] = nx.z;
         } else {
             process_cell<TERMS, SPEC>(A, S, m, r, dbg, i, mo, z, y, x, hd, ns, dtth, tr);
         }
@@ -884,6 +884,48 @@ __global__ void __launch_bounds__(384, M <= 512 ? 2 : 1) xinv4_epi_batch_kernel(
 }
 
 // ---------------------------------------------------------------- stage combine + R2C rows
+// A stage state of the block's simulation, formed cell by cell as combine_kernel forms it
+// (same operations in the same order) and written to A.next.
+struct StageCombine {
+    const float *base, *msk;
+    float* next;
+    const float* kp[MM_MAXK];
+    float ak[MM_MAXK];
+    __device__ __forceinline__ explicit StageCombine(const CombineArgs& A) {
+        const DevCtl* ctl = A.ctl + blockIdx.y;
+        const int cur = ctl->cur;
+        const long long off = blockIdx.y * A.bstride;
+        base = A.base.get(cur) + off;
+        next = A.next.get(cur) + off;
+        msk = A.msat_mask ? A.msat_mask + blockIdx.y * A.mask_bstride : nullptr;
+#pragma unroll
+        for (int j = 0; j < MM_MAXK; j++) {
+            kp[j] = j < A.nk ? A.kp[j].get(cur) + off : nullptr;
+            ak[j] = j < A.nk ? (float)(A.ak[j] * ctl->h) : 0.f;
+        }
+    }
+    __device__ __forceinline__ float3 cell(const CombineArgs& A, long long i, float& norm) const {
+        const long long N = A.N;
+        float xv = base[i], yv = base[N + i], zv = base[2 * N + i];
+#pragma unroll
+        for (int j = 0; j < MM_MAXK; j++) {
+            if (j >= A.nk) break;
+            xv += ak[j] * kp[j][i];
+            yv += ak[j] * kp[j][N + i];
+            zv += ak[j] * kp[j][2 * N + i];
+        }
+        norm = msk ? msk[i] : 1.0f;
+        const float mn = sqrtf(xv * xv + yv * yv + zv * zv);
+        float sc = (norm == 0.0f) ? 0.0f : 1.0f;
+        sc = (mn != 0.0f) ? sc / mn : 0.0f;
+        const float3 nx = make_float3(xv * sc, yv * sc, zv * sc);
+        next[i] = nx.x;
+        next[N + i] = nx.y;
+        next[2 * N + i] = nx.z;
+        return nx;
+    }
+};
+
 // The first stage state of an attempt, formed as combine_kernel forms it (same operations
 // in the same order), written to A.next and, times the Msat mask when fwd_mask, turned
 // into its R2C rows in the spectrum: the attempt's first evaluation then starts at its
@@ -897,46 +939,20 @@ __global__ void __launch_bounds__(384) combine_rows_kernel(CombineArgs A, int n0
     using F = FS<M>;
     const DevCtl* ctl = A.ctl + blockIdx.y;
     if (ctl->done) return;
-    const int cur = ctl->cur;
-    const long long off = blockIdx.y * A.bstride;
-    const float* base = A.base.get(cur) + off;
-    float* next = A.next.get(cur) + off;
-    const float* msk = A.msat_mask ? A.msat_mask + blockIdx.y * A.mask_bstride : nullptr;
-    const float* kp[MM_MAXK];
-    float ak[MM_MAXK];
-#pragma unroll
-    for (int j = 0; j < MM_MAXK; j++) {
-        kp[j] = j < A.nk ? A.kp[j].get(cur) + off : nullptr;
-        ak[j] = j < A.nk ? (float)(A.ak[j] * ctl->h) : 0.f;
-    }
+    const StageCombine C(A);
     extern __shared__ unsigned char smem_raw[];
     float2* sm = reinterpret_cast<float2*>(smem_raw);
     float* slots = reinterpret_cast<float*>(sm);
     float2* twt = sm + RPB * 3 * F::LBUF;
     F::fill_twiddles(twt, tw);
-    const long long N = A.N;
     const int nrows = n0 * n1;
     const int row0 = blockIdx.x * RPB;
     const int here = min(RPB, nrows - row0);
     for (int e = threadIdx.x; e < here * n2; e += blockDim.x) {
         const int lrow = e / n2, x = e - lrow * n2;
         const long long i = (long long)(row0 + lrow) * n2 + x;
-        float xv = base[i], yv = base[N + i], zv = base[2 * N + i];
-#pragma unroll
-        for (int j = 0; j < MM_MAXK; j++) {
-            if (j >= A.nk) break;
-            xv += ak[j] * kp[j][i];
-            yv += ak[j] * kp[j][N + i];
-            zv += ak[j] * kp[j][2 * N + i];
-        }
-        const float norm = msk ? msk[i] : 1.0f;
-        const float mn = sqrtf(xv * xv + yv * yv + zv * zv);
-        float sc = (norm == 0.0f) ? 0.0f : 1.0f;
-        sc = (mn != 0.0f) ? sc / mn : 0.0f;
-        const float3 nx = make_float3(xv * sc, yv * sc, zv * sc);
-        next[i] = nx.x;
-        next[N + i] = nx.y;
-        next[2 * N + i] = nx.z;
+        float norm;
+        const float3 nx = C.cell(A, i, norm);
         const float fm = fwd_mask ? norm : 1.0f;
         float* fl = slots + 2 * (long long)(lrow * 3) * F::LBUF + x;
         fl[0] = nx.x * fm;
@@ -993,9 +1009,13 @@ static cudaError_t launch_combine_rows_t(const CombineArgs& A, const int n[3], f
                       n[1], n[2], S, hp, L1, spec_bstride, tw, fwd_mask, RPB);
 }
 
+static cudaError_t launch_mr_combine_rows(int M, const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
+                                          long long spec_bstride, int fwd_mask, int nsim, cudaStream_t st);
+
 cudaError_t launch_combine_rows(int M, const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
                                 long long spec_bstride, const float2* tw, int fwd_mask, int nsim, cudaStream_t st) {
     if (A.no_norm || A.nk > MM_MAXK) return cudaErrorInvalidValue;
+    if (!mr_pow2(M)) return launch_mr_combine_rows(M, A, n, S, hp, L1, spec_bstride, fwd_mask, nsim, st);
     switch (M) {
 #define X(m) case m: return launch_combine_rows_t<m>(A, n, S, hp, L1, spec_bstride, tw, fwd_mask, nsim, st);
         X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024)
@@ -1289,12 +1309,37 @@ static cudaError_t launch_xinv_t(const float2* S, int hp, int L1, const float2* 
 }
 
 // ---------------------------------------------------------------- mixed-radix C2R + epilogue
+// R2C rows from transposed lines whose float x (element x/2, part x mod 2) holds the input at
+// cell x < n2; line 3*lrow + c is row row0 + lrow of component c.  Called by the whole block.
+__device__ __forceinline__ void staged_rows_r2c(const ColPlan& P, float2* sm, const unsigned short* slot,
+                                                const float2* __restrict__ twM, const float2* __restrict__ tw2M,
+                                                int row0, int lines, int n0, int n1, int n2, float2* S, int hp,
+                                                int L1) {
+    const int TC = 1 << P.sh;
+    for (int i = threadIdx.x; i < (P.N - n2 / 2) * TC; i += blockDim.x) {
+        const int e = n2 / 2 + (i >> P.sh);
+        float2* q = sm + e * P.pitch + (i & (TC - 1));
+        if (2 * e < n2) q->y = 0.f;
+        else *q = make_float2(0.f, 0.f);
+    }
+    __syncthreads();
+    lines_fft<-1>(P, sm, twM);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    for (int l = warp; l < lines; l += nw) {
+        const int row = row0 + l / 3, c = l % 3;
+        const int z = row / n1, y = row - z * n1;
+        r2c_line(P, sm + l, slot, tw2M, lane, S + ((long long)(c * n0 + z) * L1 + y) * hp);
+    }
+}
+
 // Row lengths M that are not powers of two: rpb rows of three component lines side by side
 // in shared memory (colmix.cuh), a warp per spectrum row for the pre-processing, the in-place
 // inverse, then the same epilogue.  BATCH: the simulation's scalars are staged in shared
 // memory (batched plans, time tables).
-template <bool TERMS, bool BATCH, int SPEC>
-__global__ void __launch_bounds__(384, 2) mr_xinv_epi_kernel(const float2* __restrict__ S, int hp, int L1,
+// FWD: then the R2C rows of the next stage state into the spectrum rows just read, as
+// mr_rows_kernel makes them.
+template <bool TERMS, bool BATCH, bool FWD, int SPEC>
+__global__ void __launch_bounds__(384, 2) mr_xinv_epi_kernel(typename SpecIn<FWD>::type S, int hp, int L1,
                                                           const __grid_constant__ ColPlan P,
                                                           const float2* __restrict__ twM,
                                                           const float2* __restrict__ tw2M, EpiArgs A, int rpb) {
@@ -1321,8 +1366,42 @@ __global__ void __launch_bounds__(384, 2) mr_xinv_epi_kernel(const float2* __res
     }
     __syncthreads();
     lines_fft<+1>(P, sm, twM);
-    epilogue_rows<TERMS, false, BATCH, false, SPEC, true>(A, pick_scalars<BATCH>(s_sim, A.P.s), sm, P.pitch, row0,
-                                                          here);
+    epilogue_rows<TERMS, false, BATCH, FWD, SPEC, true>(A, pick_scalars<BATCH>(s_sim, A.P.s), sm, P.pitch, row0, here);
+    if constexpr (FWD) {
+        __syncthreads();
+        staged_rows_r2c(P, sm, slot, twM, tw2M, row0, 3 * here, n0, n1, A.P.n[2],
+                        A.fwd + blockIdx.y * A.spec_bstride, hp, L1);
+    }
+}
+
+// combine_rows_kernel for these row lengths: the attempt's first stage state and its R2C rows.
+__global__ void __launch_bounds__(384, 2) mr_combine_rows_kernel(CombineArgs A, int n0, int n1, int n2, float2* S,
+                                                                 int hp, int L1, long long spec_bstride,
+                                                                 const __grid_constant__ ColPlan P,
+                                                                 const float2* __restrict__ twM,
+                                                                 const float2* __restrict__ tw2M, int fwd_mask,
+                                                                 int rpb) {
+    pdl_begin();
+    if (A.ctl[blockIdx.y].done) return;
+    extern __shared__ unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+    unsigned short* slot = reinterpret_cast<unsigned short*>(sm + P.N * P.pitch);
+    fill_slots(P, slot);
+    const int row0 = (int)blockIdx.x * rpb, here = min(rpb, n0 * n1 - row0);
+    const StageCombine C(A);
+    float* fl = reinterpret_cast<float*>(sm);
+    for (int e = threadIdx.x; e < here * n2; e += blockDim.x) {
+        const int lrow = e / n2, x = e - lrow * n2;
+        float norm;
+        const float3 nx = C.cell(A, (long long)row0 * n2 + e, norm);
+        const float fm = fwd_mask ? norm : 1.0f;
+        float* q = fl + 2 * ((x >> 1) * P.pitch + lrow * 3) + (x & 1);
+        q[0] = nx.x * fm;
+        q[2] = nx.y * fm;
+        q[4] = nx.z * fm;
+    }
+    __syncthreads();
+    staged_rows_r2c(P, sm, slot, twM, tw2M, row0, 3 * here, n0, n1, n2, S + blockIdx.y * spec_bstride, hp, L1);
 }
 
 // Rows per block (5, 2 or 1: three lines each of 16, 8 or 4) and threads of the mixed-radix
@@ -1338,7 +1417,27 @@ static void mr_xinv_shape(int M, int n0n1, int n2, int nsim, int* rpb, int* sh, 
     *threads = std::max(96, ((cells + turns - 1) / turns + 31) / 32 * 32);
 }
 
-template <bool TERMS, bool BATCH>
+static cudaError_t launch_mr_combine_rows(int M, const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
+                                          long long spec_bstride, int fwd_mask, int nsim, cudaStream_t st) {
+    ColPlan P;
+    const float2 *twM = nullptr, *tw2M = nullptr;
+    if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !mr_tables(2 * M, &tw2M, nullptr))
+        return cudaErrorInvalidValue;
+    int rpb, threads;
+    mr_xinv_shape(M, n[0] * n[1], n[2], nsim, &rpb, &P.sh, &threads);
+    P.pitch = (1 << P.sh) + 1;
+    const size_t smem = lines_smem(M, 1 << P.sh);
+    if (smem > 48 * 1024) {
+        const cudaError_t e =
+            cudaFuncSetAttribute(mr_combine_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const int blocks = (n[0] * n[1] + rpb - 1) / rpb;
+    return launch_pdl(mr_combine_rows_kernel, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, A, n[0],
+                      n[1], n[2], S, hp, L1, spec_bstride, P, twM, tw2M, fwd_mask, rpb);
+}
+
+template <bool TERMS, bool BATCH, bool FWD>
 static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, const EpiArgs& A, cudaStream_t st,
                                     int* nblocks, int nsim) {
     ColPlan P;
@@ -1350,15 +1449,15 @@ static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, cons
     P.pitch = (1 << P.sh) + 1;
     const size_t smem = lines_smem(M, 1 << P.sh);
     // the epilogue without what the evaluation lacks (as the four-step pass chooses it)
-    auto kern = mr_xinv_epi_kernel<TERMS, BATCH, 0>;
+    auto kern = mr_xinv_epi_kernel<TERMS, BATCH, FWD, 0>;
     if constexpr (!TERMS) {
         const int spec = epilogue_spec(A.P);
         constexpr int NOTS = SPEC_NOTHERMAL | SPEC_NOSTT, NOMS = SPEC_NOMASK | SPEC_NOSTT,
                       NOMT = SPEC_NOMASK | SPEC_NOTHERMAL;
-        if (spec == SPEC_LEAN) kern = mr_xinv_epi_kernel<false, BATCH, SPEC_LEAN>;
-        else if ((spec & NOTS) == NOTS) kern = mr_xinv_epi_kernel<false, BATCH, NOTS>;
-        else if ((spec & NOMS) == NOMS) kern = mr_xinv_epi_kernel<false, BATCH, NOMS>;
-        else if ((spec & NOMT) == NOMT) kern = mr_xinv_epi_kernel<false, BATCH, NOMT>;
+        if (spec == SPEC_LEAN) kern = mr_xinv_epi_kernel<false, BATCH, FWD, SPEC_LEAN>;
+        else if ((spec & NOTS) == NOTS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOTS>;
+        else if ((spec & NOMS) == NOMS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMS>;
+        else if ((spec & NOMT) == NOMT) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMT>;
     }
     if (smem > 48 * 1024) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1473,9 +1572,9 @@ X(1024)
 
 static bool use_xinv4(int M) { return M >= 4 && M <= 1024 && mr_pow2(M); }
 
-// The four-step epilogue (and the four-step row pass whose output it reproduces) serve
-// these row lengths.
-bool epi_r2c_supported(int M) { return use_xinv4(M); }
+// The row lengths whose epilogue can write the next stage's R2C rows: the four-step one and
+// the mixed-radix one (each reproduces its row pass).
+bool epi_r2c_supported(int M) { return use_xinv4(M) || !mr_pow2(M); }
 
 // The most blocks per simulation that the pass may take for n0n1 rows (the size of the
 // reduction partials).
@@ -1502,11 +1601,17 @@ cudaError_t launch_xinv_epi(int M, const float2* S, int hp, int L1, const float2
         }
     }
     if (!mr_pow2(M)) {  // not a power of two: the mixed-radix pass
-        if (staged)
-            return terms ? launch_mr_xinv_t<true, true>(M, S, hp, L1, A, st, nblocks, nsim)
-                         : launch_mr_xinv_t<false, true>(M, S, hp, L1, A, st, nblocks, nsim);
-        return terms ? launch_mr_xinv_t<true, false>(M, S, hp, L1, A, st, nblocks, 1)
-                     : launch_mr_xinv_t<false, false>(M, S, hp, L1, A, st, nblocks, 1);
+        const int ns = staged ? nsim : 1;
+        if (terms) {
+            if (A.fwd) return cudaErrorInvalidValue;
+            return staged ? launch_mr_xinv_t<true, true, false>(M, S, hp, L1, A, st, nblocks, ns)
+                          : launch_mr_xinv_t<true, false, false>(M, S, hp, L1, A, st, nblocks, ns);
+        }
+        if (A.fwd)
+            return staged ? launch_mr_xinv_t<false, true, true>(M, S, hp, L1, A, st, nblocks, ns)
+                          : launch_mr_xinv_t<false, false, true>(M, S, hp, L1, A, st, nblocks, ns);
+        return staged ? launch_mr_xinv_t<false, true, false>(M, S, hp, L1, A, st, nblocks, ns)
+                      : launch_mr_xinv_t<false, false, false>(M, S, hp, L1, A, st, nblocks, ns);
     }
     if (staged) return cudaErrorNotSupported;  // batched plans and time tables use the four-step pass
     switch (M) {
