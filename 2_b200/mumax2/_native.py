@@ -193,6 +193,8 @@ _PROTOS = {
                             C.c_void_p, C.c_void_p]),
     "mm_nn_adam": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_longlong, C.c_float, C.c_float,
                              C.c_float, C.c_float, C.c_int, C.c_void_p, C.c_void_p]),
+    "mm_nn_adam_net": (C.c_int, [C.c_void_p] * 6 + [C.c_int] + [C.POINTER(C.c_int)] * 4 + [C.c_float] * 4 +
+                       [C.c_int, C.c_void_p]),
     "mm_nn_flip": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_int, C.c_void_p]),
     "mm_nn_output_state": (C.c_int, [C.c_void_p, C.c_int, C.c_void_p, C.c_longlong, C.c_int, C.c_void_p,
                                      C.c_void_p]),

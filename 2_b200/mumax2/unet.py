@@ -153,20 +153,30 @@ class UNet:
             npx = batch * (H >> lvl) * (W >> lvl)
             self.buf[k] = torch.zeros(npx * ch, dtype=bf, device=self.device)
             self.grad[k] = torch.zeros(npx * ch, dtype=bf, device=self.device)
+        # every layer's weights back to back, then the biases: one launch updates them all
         self.p = {}
         params = params or init_params(seed)
-        for name, _, cin, _, cout, _ in CONVS:
-            w, b = params[name]
-            d = {"w": torch.tensor(w, device=self.device).reshape(-1), "b": torch.tensor(b, device=self.device)}
-            d["wb"] = d["w"].to(bf)
-            cin_t = ((cout + 15) // 16) * 16
-            d["wt"] = torch.zeros(cin * 9 * cin_t, dtype=bf, device=self.device)
-            d["cin_t"] = cin_t
-            for k in ("gw", "mw", "vw"):
-                d[k] = torch.zeros_like(d["w"])
-            for k in ("gb", "mb", "vb"):
-                d[k] = torch.zeros_like(d["b"])
+        nw = [c[4] * 9 * c[2] for c in CONVS]
+        cin_t = [((c[4] + 15) // 16) * 16 for c in CONVS]
+        nt = [c[2] * 9 * t for c, t in zip(CONVS, cin_t)]
+        host = np.concatenate([params[c[0]][k].ravel() for k in (0, 1) for c in CONVS]).astype(np.float32)
+        flat = {"w": torch.tensor(host, device=self.device)}
+        for k in ("g", "m", "v"):
+            flat[k] = torch.zeros_like(flat["w"])
+        flat["wb"] = flat["w"][:sum(nw)].to(bf)
+        flat["wt"] = torch.zeros(sum(nt), dtype=bf, device=self.device)
+        self.flat = flat
+        ow, ob, ot = 0, sum(nw), 0
+        for (name, _, _, _, cout, _), n, ct, n_t in zip(CONVS, nw, cin_t, nt):
+            d = {"cin_t": ct, "wb": flat["wb"][ow:ow + n], "wt": flat["wt"][ot:ot + n_t]}
+            for k, f in (("", "w"), ("g", "g"), ("m", "m"), ("v", "v")):
+                d[k + "w"], d[k + "b"] = flat[f][ow:ow + n], flat[f][ob:ob + cout]
             self.p[name] = d
+            ow, ob, ot = ow + n, ob + cout, ot + n_t
+        ints = lambda v: (C.c_int * len(v))(*v)  # noqa: E731
+        # the last layer's unused output rows stay zero
+        self._layers = (len(CONVS), ints([c[4] for c in CONVS]), ints([c[2] for c in CONVS]), ints(cin_t),
+                        ints([3 if c[0] == "out" else c[4] for c in CONVS]))
         self.t = 0
         self.target = None
         self.mask = None
@@ -287,9 +297,7 @@ class UNet:
         B, H, W = self.B, self.H, self.W
         convs = {c[0]: c for c in CONVS}
         fp = self._ptr
-        for d in self.p.values():
-            d["gw"].zero_()
-            d["gb"].zero_()
+        self.flat["g"].zero_()
         for op in reversed(SCHEDULE):
             if op.startswith("pool"):
                 (sv, so), (dv, do), ch, lvl = POOLS[int(op[4:])]
@@ -321,20 +329,10 @@ class UNet:
                                self._cs((iv,)), io, cin, H >> lvl, W >> lvl, 0)
 
     def adam(self, lr=1e-3, b1=0.9, b2=0.999, eps=1e-8):
-        L = nat.lib()
         self.t += 1
-        fp = self._ptr
-        for name, d in self.p.items():
-            nat.check(L.mm_nn_adam(fp(d["w"]), fp(d["gw"]), fp(d["mw"]), fp(d["vw"]), d["w"].numel(), C.c_float(lr),
-                                   C.c_float(b1), C.c_float(b2), C.c_float(eps), self.t, self._ptr(d["wb"]), None))
-            nat.check(L.mm_nn_adam(fp(d["b"]), fp(d["gb"]), fp(d["mb"]), fp(d["vb"]), d["b"].numel(), C.c_float(lr),
-                                   C.c_float(b1), C.c_float(b2), C.c_float(eps), self.t, None, None))
-        # the last layer's unused output rows stay zero
-        dl = self.p["out"]
-        w = dl["w"].reshape(OUTC, -1)
-        w[3:].zero_()
-        dl["wb"].copy_(dl["w"].to(self.torch.bfloat16))
-        self._flip_all()
+        f = self.flat
+        nat.check(nat.lib().mm_nn_adam_net(*(self._ptr(f[k]) for k in ("w", "g", "m", "v", "wb", "wt")), *self._layers,
+                                           lr, b1, b2, eps, self.t, None))
 
     def states(self, masks_dev, dst):
         """Initial states of this batch from the output: dst (float32 device tensor

@@ -362,6 +362,14 @@ MM_API int mm_nn_mse(const void* out, int o_cs, const float* target, const float
 MM_API int mm_nn_adam(float* w, const float* g, float* m, float* v, long long n, float lr, float b1, float b2,
                       float eps, int t, void* wb, mm_stream st);
 MM_API int mm_nn_flip(const void* W, int Cout, int Cin, void* Wt, int Cin_t, int Cout_t, mm_stream st);
+/* mm_nn_adam and mm_nn_flip over a whole network of up to 16 layers: w, g, m, v hold the layers'
+ * weights [cout][9][cin] back to back, then their biases; wb (bf16) the weights' copies, wt
+ * (bf16) the flipped copies [cin][9][cin_t] back to back.  Weight rows from live[l] on of layer
+ * l are set to zero. */
+#define MM_NN_MAX_LAYERS 16
+MM_API int mm_nn_adam_net(float* w, const float* g, float* m, float* v, void* wb, void* wt, int nlayers,
+                          const int* cout, const int* cin, const int* cin_t, const int* live, float lr, float b1,
+                          float b2, float eps, int t, mm_stream st);
 /* warm-start input features [nq][P][16] bf16 from masks [nq][P] and prm [nq][8] =
  * (Ms, Aex, Ku1, axis x, axis y, B_x, B_y, 0) in user axes (see unet.py). */
 MM_API int mm_nn_features(const float* masks, const float* prm, long long nq, int P, void* out, mm_stream st);

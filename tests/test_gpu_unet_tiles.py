@@ -1,6 +1,6 @@
-"""The tcgen05 convolution with several position tiles per block and the weight gradient's ring
-of positions, at the sizes where their tiles change; against float64 sums by torch of the same
-bf16 values."""
+"""The tcgen05 convolution with several position tiles per block, the weight gradient's ring of
+positions, and the whole-network optimiser step, at the sizes where their tiles change; against
+float64 sums by torch of the same bf16 values."""
 import ctypes as C
 
 import pytest
@@ -57,3 +57,30 @@ def test_weight_gradient_ring(cin, cout, B, H, W, shift):
     ref = torch.stack([dy.double().t() @ v for v in _taps(x, B, H, W, cin)], 1).reshape(-1)
     # FP32 sums of P products in a few hundred partial sums: eps * sqrt(P) of the norm and more
     assert float((dw.double() - ref).norm() / ref.norm()) < 1e-5
+
+
+def test_network_step_equals_layer_steps():
+    """mm_nn_adam_net against mm_nn_adam and mm_nn_flip per layer, bit for bit."""
+    import torch
+    from mumax2 import _native as nat
+    from mumax2 import unet as U
+    net = U.UNet(2, H=16, W=16, seed=3)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    for _ in range(2):
+        net.flat["g"].copy_(torch.randn(net.flat["g"].numel(), device="cuda", generator=g))
+        want = {}
+        for name, _, cin, _, cout, _ in U.CONVS:
+            d = net.p[name]
+            q = {k: d[k].clone() for k in ("w", "gw", "mw", "vw", "wb", "b", "gb", "mb", "vb", "wt")}
+            for k, wb in (("w", _p(q["wb"])), ("b", None)):
+                nat.check(nat.lib().mm_nn_adam(_p(q[k]), _p(q["g" + k]), _p(q["m" + k]), _p(q["v" + k]), q[k].numel(),
+                                               1e-2, 0.9, 0.999, 1e-8, net.t + 1, wb, None))
+            if name == "out":
+                q["w"].reshape(cout, -1)[3:].zero_()
+                q["wb"].copy_(q["w"].to(torch.bfloat16))
+            nat.check(nat.lib().mm_nn_flip(_p(q["wb"]), cout, cin, _p(q["wt"]), d["cin_t"], cin, None))
+            want[name] = q
+        net.adam(lr=1e-2)
+        for name, q in want.items():
+            for k, v in q.items():
+                assert torch.equal(net.p[name][k], v), (name, k)
