@@ -988,11 +988,12 @@ static cudaError_t launch_colmul4_t(float2* S, const KernelView& K, int ncols, l
                                     long long line_stride, int n_in, float scale, const float2* tw,
                                     const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
                                     long long sim_stride, const float* sim_scale, int tile) {
-    // single small films: fewer columns per block while the blocks leave SMs idle (a 128x32
-    // film has 129 columns, 17 blocks of the default 8)
+    // single small films of up to 64 rows: fewer columns per block while the blocks leave SMs
+    // idle (a 128x32 film has 129 columns, 17 blocks of the default 8).  Longer columns keep
+    // their tile: 48-thread blocks of one 256-point column take 11.1 us, 192-thread ones 10.0.
     int shift = tile;
     const long long cols = (long long)ncols * nsim;
-    while (shift > -3 && cols < 148LL * (64 / FS<L>::P2 >> -std::min(shift, 0))) shift--;
+    while (L <= 128 && shift > -3 && cols < 148LL * (64 / FS<L>::P2 >> -std::min(shift, 0))) shift--;
 #define GO(sh)                                                                                                  \
     return launch_colmul4_s<L, sh, false>(S, K, ncols, 1, comp_stride, 0, line_stride, n_in, scale, tw, ctl,    \
                                           skip_retry, st, nsim, sim_stride, sim_scale)
