@@ -501,8 +501,12 @@ __global__ void relu_bwd_kernel(const bf16* out, int o_cs, int o_co, bf16* d, in
 // of a pixel (16-byte loads; consecutive threads cover consecutive channels, then the
 // next pixels), zeroes the gradient where the forward output was not positive (relu),
 // keeps 8 register sums for its channels, and the block adds its per-channel sums to db.
-__global__ void relu_bias_bwd_kernel(const bf16* __restrict__ out, int o_cs, int o_co, bf16* __restrict__ d, int d_cs,
-                                     int d_co, int C, long long P, long long ppb, int relu, float* __restrict__ db) {
+// Latency-bound on its loads: four pixels of a thread are in flight at a time, and lanes of the
+// same channels (G a power of two) are summed by shuffles before the shared-memory atomics.
+__global__ void __launch_bounds__(512) relu_bias_bwd_kernel(const bf16* __restrict__ out, int o_cs, int o_co,
+                                                            bf16* __restrict__ d, int d_cs, int d_co, int C,
+                                                            long long P, long long ppb, int relu,
+                                                            float* __restrict__ db) {
     __shared__ float acc[512];
     const int G = C / 8;                       // threads per pixel
     const int K = blockDim.x / G;              // pixels per block iteration
@@ -511,32 +515,53 @@ __global__ void relu_bias_bwd_kernel(const bf16* __restrict__ out, int o_cs, int
     __syncthreads();
     const long long p0 = blockIdx.x * ppb, p1 = min(P, p0 + ppb);
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    constexpr int U = 4;
     if (r < K) {
-        for (long long p = p0 + r; p < p1; p += K) {
-            uint4* gp = reinterpret_cast<uint4*>(d + p * d_cs + d_co + 8 * g);
-            uint4 gv = *gp;
-            __nv_bfloat162* gh = reinterpret_cast<__nv_bfloat162*>(&gv);
-            if (relu) {
-                const uint4 ov = *reinterpret_cast<const uint4*>(out + p * o_cs + o_co + 8 * g);
-                const __nv_bfloat162* oh = reinterpret_cast<const __nv_bfloat162*>(&ov);
-                bool changed = false;
+        for (long long p = p0 + r; p < p1; p += (long long)U * K) {
+            uint4 gv[U], ov[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const long long q = p + (long long)u * K;
+                gv[u] = ov[u] = make_uint4(0u, 0u, 0u, 0u);
+                if (q < p1) {
+                    gv[u] = *reinterpret_cast<const uint4*>(d + q * d_cs + d_co + 8 * g);
+                    if (relu) ov[u] = *reinterpret_cast<const uint4*>(out + q * o_cs + o_co + 8 * g);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const long long q = p + (long long)u * K;
+                __nv_bfloat162* gh = reinterpret_cast<__nv_bfloat162*>(&gv[u]);
+                if (relu && q < p1) {
+                    const __nv_bfloat162* oh = reinterpret_cast<const __nv_bfloat162*>(&ov[u]);
+                    bool changed = false;
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const float2 of = __bfloat1622float2(oh[k]);
+                        float2 gf = __bfloat1622float2(gh[k]);
+                        if (!(of.x > 0.f)) { gf.x = 0.f; changed = true; }
+                        if (!(of.y > 0.f)) { gf.y = 0.f; changed = true; }
+                        gh[k] = __floats2bfloat162_rn(gf.x, gf.y);
+                    }
+                    if (changed) *reinterpret_cast<uint4*>(d + q * d_cs + d_co + 8 * g) = gv[u];
+                }
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
-                    const float2 of = __bfloat1622float2(oh[k]);
-                    float2 gf = __bfloat1622float2(gh[k]);
-                    if (!(of.x > 0.f)) { gf.x = 0.f; changed = true; }
-                    if (!(of.y > 0.f)) { gf.y = 0.f; changed = true; }
-                    gh[k] = __floats2bfloat162_rn(gf.x, gf.y);
+                    const float2 gf = __bfloat1622float2(gh[k]);
+                    s[2 * k] += gf.x;
+                    s[2 * k + 1] += gf.y;
                 }
-                if (changed) *gp = gv;
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const float2 gf = __bfloat1622float2(gh[k]);
-                s[2 * k] += gf.x;
-                s[2 * k + 1] += gf.y;
             }
         }
+    }
+    bool add = r < K;
+    if ((G & (G - 1)) == 0 && G < 32 && blockDim.x % 32 == 0) {
+        for (int o = 16; o >= G; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < 8; k++) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        add = add && (threadIdx.x & 31) < G;
+    }
+    if (add) {
 #pragma unroll
         for (int k = 0; k < 8; k++) atomicAdd(&acc[8 * g + k], s[k]);
     }
