@@ -219,7 +219,10 @@ __global__ void controller_kernel(DevCtl* ctl, int nsim, CtlSummary* sum, int mo
     int active = 0, bad = 0x7fffffff;
     long long left = 0;
     for (int b = threadIdx.x; b < nsim; b += blockDim.x) {
-        DevCtl* c = ctl + b;
+        // a local copy: one round trip for the block's fields, then one for the stores, where
+        // working in place takes one for each group of fields that a branch waits for
+        DevCtl local = ctl[b];
+        DevCtl* c = &local;
         if (mode == 1) control_one(c, adaptive, q, fsal, nevals, first_skippable);
         if (mode == 2 && !c->done) {
             // run_until_smaller for non-FSAL solvers: the torque k0 of the current state is
@@ -231,6 +234,7 @@ __global__ void controller_kernel(DevCtl* ctl, int nsim, CtlSummary* sum, int mo
             }
             c->tq_bits = 0u;
         }
+        if (mode != 0) ctl[b] = local;
         if (!c->done) {
             active++;
             left = max(left, c->step_end - c->step);
