@@ -135,26 +135,11 @@ __device__ __forceinline__ void tile_load(V* sm, const V* __restrict__ base, lon
                                           int cline, bool zero) {
     constexpr int LL = line_len(L);
     const int nthr = blockDim.x;
-    bool done_vec = false;
-    if constexpr (TC >= 2 && sizeof(V) == 8) {
-        if (ncols_here == TC) {
-            constexpr int TP = TC / 2;  // two columns per 16-byte access
-            for (int i = threadIdx.x; i < n * TP; i += nthr) {
-                const int e = i / TP, cp = (i % TP) * 2;
-                float4 v = __ldg(reinterpret_cast<const float4*>(base + e * line_stride + cp));
-                sm[(cline + cp) * LL + padx(e)] = make_float2(v.x, v.y);
-                sm[(cline + cp + 1) * LL + padx(e)] = make_float2(v.z, v.w);
-            }
-            done_vec = true;
-        }
-    }
-    if (!done_vec) {
-        for (int i = threadIdx.x; i < n * TC; i += nthr) {
-            const int e = i / TC, col = i % TC;
-            V v = mkv((typename Scalar<V>::T)0, (typename Scalar<V>::T)0);
-            if (col < ncols_here) v = base[e * line_stride + col];
-            sm[(cline + col) * LL + padx(e)] = v;
-        }
+    for (int i = threadIdx.x; i < n * TC; i += nthr) {
+        const int e = i / TC, col = i % TC;
+        V v = mkv((typename Scalar<V>::T)0, (typename Scalar<V>::T)0);
+        if (col < ncols_here) v = base[e * line_stride + col];
+        sm[(cline + col) * LL + padx(e)] = v;
     }
     if (zero) {
         for (int i = threadIdx.x; i < (L - n) * TC; i += nthr) {
@@ -169,24 +154,9 @@ __device__ __forceinline__ void tile_store(const V* sm, V* __restrict__ base, lo
                                            int cline) {
     constexpr int LL = line_len(L);
     const int nthr = blockDim.x;
-    bool done_vec = false;
-    if constexpr (TC >= 2 && sizeof(V) == 8) {
-        if (ncols_here == TC) {
-            constexpr int TP = TC / 2;
-            for (int i = threadIdx.x; i < n * TP; i += nthr) {
-                const int e = i / TP, cp = (i % TP) * 2;
-                V a = sm[(cline + cp) * LL + padx(e)];
-                V b = sm[(cline + cp + 1) * LL + padx(e)];
-                *reinterpret_cast<float4*>(base + e * line_stride + cp) = make_float4(a.x, a.y, b.x, b.y);
-            }
-            done_vec = true;
-        }
-    }
-    if (!done_vec) {
-        for (int i = threadIdx.x; i < n * TC; i += nthr) {
-            const int e = i / TC, col = i % TC;
-            if (col < ncols_here) base[e * line_stride + col] = sm[(cline + col) * LL + padx(e)];
-        }
+    for (int i = threadIdx.x; i < n * TC; i += nthr) {
+        const int e = i / TC, col = i % TC;
+        if (col < ncols_here) base[e * line_stride + col] = sm[(cline + col) * LL + padx(e)];
     }
 }
 
@@ -238,7 +208,8 @@ __device__ __forceinline__ float2 wtab(const float2* __restrict__ tw, int m, int
 
 // BATCH: the block does `group` simulations one after the other with its columns' kernel
 // values in registers: they are the same for all, and with one simulation per block their 6 P
-// gathers per lane are twice the spectrum's 3 P loads.
+// gathers per lane are twice the spectrum's 3 P loads (103 simulations of 128x128x4 cells:
+// 257 -> 169 us).  Bound by the spectrum's round trip through L2 and HBM.
 template <int P, bool BATCH>
 __global__ void __launch_bounds__(128) zmul_reg_kernel(float2* __restrict__ S, KernelView K, int L1, int h, int hp,
                                                        long long comp_stride, long long zstride, float scale,
@@ -486,7 +457,8 @@ cudaError_t launch_zmul_reg(int P, float2* S, const KernelView& K, int L1, int h
     }
     switch (P) {
 #define X(p, f) case p: return f<p>(S, K, L1, h, hp, comp_stride, zstride, scale, tw, tws, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
-        // two lanes per column up to P = 15 (measured: P = 4, 128x128x4 ensemble class
+        // two lanes per column up to P = 15 (P = 3, 150x75x3 body: 5.5 us, where the columns in
+        // shared memory took 46; measured besides: P = 4, 128x128x4 ensemble class
         // 1073 -> 1012 us; P = 8, 8x128x128 film 11.8 -> 11.0 us), four at P = 16
         X(1, launch_zmul_reg_t) X(2, launch_zmul_reg_t) X(3, launch_zmul_reg_t) X(4, launch_zmul_reg_t)
         X(5, launch_zmul_reg_t) X(6, launch_zmul_reg_t) X(7, launch_zmul_reg_t) X(8, launch_zmul_reg_t)
@@ -641,7 +613,7 @@ __global__ void __launch_bounds__(512) xfwd4_kernel(const float* __restrict__ in
 // three components of a (ky, kx) point meet in one thread), taken back into registers
 // and inverse-transformed; only the rows n < n_in are stored.  ZAX: lines along z of bodies too
 // tall for the register multiply, one (ky, kx tile) per block.  Replaces the Stockham
-// colmul_kernel for 2-D films (seven barrier-separated stages per transform and
+// Stockham pass for 2-D films (seven barrier-separated stages per transform and
 // component there, two barriers per transform here).
 template <int L, int TC, bool ZAX>
 __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, KernelView K, int ncols,
@@ -719,7 +691,9 @@ __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, Ke
 // exchange buffers at 2H: by the parity of the frequency, X[2k] = DFT_H(x)[k] and
 // X[2k+1] = DFT_H(x W_2H^n)[k], one after the other; the inverse's first H rows are the sum of
 // the two inverses, the odd one times W_2H^-n, kept in registers.  The input is read twice (the
-// second time from L2) and written at the end.
+// second time from L2) and written at the end.  Four columns (32-byte rows) and 101 KB per
+// block, one block per SM by its registers; bound by the barriers between its phases with 12
+// warps: 91 us for 1024x1024 cells, where all 2048 frequencies at once took 156.
 template <int H, int TC>
 __global__ void __launch_bounds__(3 * TC * FS<H>::P2, 1) colmul_split_kernel(
     float2* __restrict__ S, KernelView K, int ncols, long long comp_stride, long long line_stride, int n_in, float scale,
@@ -1022,7 +996,7 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
         }
     }
     if (kaxis == 0) {
-        // tall bodies: the four-step pass along z
+        // tall bodies: the four-step pass along z (64^3 cells: 45 us; Stockham stages 81)
         switch (L) {
 #define X(l) case l: return launch_colmul4_s<l, 0, true>(S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
             X(8) X(16) X(32) X(64) X(128) X(256) X(512)

@@ -2,11 +2,11 @@
 //
 // Same passes, spectrum layout and arithmetic as the power-of-two kernels of conv.cu
 // (R2C rows by the packed half-length transform, column transforms of the non-zero
-// rows only, the symmetric 3x3 kernel multiply between forward and inverse), with the
-// transform itself done by the mixed-radix shared-memory routine of mixed.cuh.  Used
+// rows only).  The FP32 rows use the in-place stages of colmix.cuh (the columns are in
+// colmix.cu, the C2R + epilogue pass in rhs.cu, mr_xinv_epi_kernel); the FP64 transform of
+// the demag tensor at plan creation uses the shared-memory routine of mixed.cuh.  Used
 // for padded sizes such as 2^n * {3, 5, 7} (engine/gridsize.go:16-33), which the
-// reference convolves through cuFFT (fftplanX.go:59-64).  The C2R + epilogue pass of
-// these lengths is in rhs.cu (mr_xinv_epi_kernel).
+// reference convolves through cuFFT (fftplanX.go:59-64).
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -191,7 +191,9 @@ cudaError_t launch_mr_xfwd(int M, const S* in, PP pp, const float* mask, V* out,
 
 // The FP32 row pass: TC rows per block side by side in shared memory (colmix.cuh), a warp per
 // row between global memory and the transposed lines (pitch TC + 1: consecutive elements of
-// a row fall on distinct banks).
+// a row fall on distinct banks).  With the epilogue in the same form, 192x192x8 cells, RK12
+// step 253 -> 219 us; latency-bound.  Natural order through a second buffer instead of the slot
+// table took 1 % more (half the lines per SM).
 __global__ void __launch_bounds__(256, 3) mr_rows_kernel(const float* __restrict__ in_fixed, PP in_pp,
                                                          const float* __restrict__ mask, float2* __restrict__ out,
                                                          int nrows, int Z, int Y, int Yout, int in_pitch, int n_in,

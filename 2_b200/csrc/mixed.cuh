@@ -4,7 +4,8 @@
 // The reference accepts any padded size (cuFFT, fftplanX.go:59-64) and recommends
 // 2^n * {1, 3, 5, 7} (engine/gridsize.go:16-33).  The power-of-two passes (fft.cuh,
 // fft4.cuh) serve the common case; every other length L <= 4096 whose prime factors are
-// at most MR_MAXR goes through these routines: a self-sorting Stockham transform
+// at most MR_MAXR goes through the stages of colmix.cuh in FP32 and, for the FP64 transform
+// of the demag tensor, through these routines: a self-sorting Stockham transform
 // (Govindaraju et al., SC'08; natural-order output, no bit reversal) with one stage per
 // factor, radices 8, 4, 2 in registers and every other prime factor as a direct DFT.
 // Twiddles come from per-length tables of exp(-2 pi i t / L), computed in FP64 on the
