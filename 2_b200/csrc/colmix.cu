@@ -301,11 +301,6 @@ bool radix_search(int n, int left, int most, int cap, int* out, int depth, int* 
     return false;
 }
 
-template <typename KT> cudaError_t mc_smem(KT kern, size_t bytes) {
-    if (bytes > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return cudaSuccess;
-}
-
 // Columns per block: 16 (128-byte rows) while the lines fit 48 KB, fewer for longer lines
 // (2 at most 200 KB) and for grids of less than one block per SM.
 int pick_cols(size_t line_bytes, int ncols, long long outer) {
@@ -371,7 +366,7 @@ cudaError_t launch_colmix_fft(int L, int sign, float2* S, int ncols, int nouter,
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
     cudaError_t e;
     auto kern = sign < 0 ? colmix_fft_kernel<-1> : colmix_fft_kernel<1>;
-    if ((e = mc_smem(kern, smem)) != cudaSuccess) return e;
+    if ((e = allow_smem(kern, smem)) != cudaSuccess) return e;
     return launch_pdl(kern, grid, dim3(threads), smem, st, S, ncols, outer_stride, line_stride, n_in, n_out, P, tw, ctl,
                       skip_retry, sim_stride);
 }
@@ -394,7 +389,7 @@ cudaError_t launch_colmix_mul(int L, float2* S, const KernelView& K, int ncols, 
     const int threads = pick_threads(std::max(P.NP * P.nq, 3 * P.N / P.r[0]) * tc);
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
     cudaError_t e;
-    if ((e = mc_smem(colmix_mul_kernel, smem)) != cudaSuccess) return e;
+    if ((e = allow_smem(colmix_mul_kernel, smem)) != cudaSuccess) return e;
     return launch_pdl(colmix_mul_kernel, grid, dim3(threads), smem, st, S, K, ncols, comp_stride, outer_stride,
                       line_stride, n_in, kaxis, scale, P, tw, ctl, skip_retry, sim_stride, sim_scale);
 }

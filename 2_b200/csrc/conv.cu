@@ -770,11 +770,6 @@ __global__ void __launch_bounds__(3 * TC * FS<H>::P2, 1) colmul_split_kernel(
 }
 
 // ---------------------------------------------------------------- launch helpers
-template <typename KT> static cudaError_t set_smem(KT kern, size_t bytes) {
-    if (bytes > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return cudaSuccess;
-}
-
 #define MM_FOR_POW2(X) X(1) X(2) X(4) X(8) X(16) X(32) X(64) X(128) X(256) X(512) X(1024) X(2048) X(4096)
 
 #define XFWD_SIM_ARGS int nsim, long long in_bstride, long long out_bstride, long long mask_bstride
@@ -787,7 +782,7 @@ static cudaError_t launch_xfwd_t(const S* in, PP pp, const float* mask, V* out, 
     constexpr int TPL = tpl(M);
     constexpr int RPB = TPL >= 256 ? 1 : 256 / TPL;
     const size_t smem = (size_t)RPB * line_len(M) * sizeof(V);
-    cudaError_t e = set_smem(xfwd_kernel<M, V, S>, smem);
+    cudaError_t e = allow_smem(xfwd_kernel<M, V, S>, smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((nrows + RPB - 1) / RPB), (unsigned)nsim);
     int threads = RPB * TPL < 32 ? 32 : RPB * TPL;
@@ -806,7 +801,7 @@ static cudaError_t launch_xfwd4_t(const float* in, PP pp, const float* mask, flo
     int RPB = shifted(RPB0, tile);
     if (RPB < 1 || RPB * F::P2 > 512 || RPB * F::P2 < 32 || smem_of(RPB) > 200 * 1024) RPB = RPB0;
     const size_t smem = smem_of(RPB);
-    cudaError_t e = set_smem(xfwd4_kernel<M>, smem);
+    cudaError_t e = allow_smem(xfwd4_kernel<M>, smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((nrows + RPB - 1) / RPB), (unsigned)nsim);
     return launch_pdl(xfwd4_kernel<M>, grid, dim3(RPB * F::P2), smem, st, in, pp, mask, out, nrows, Z, Y, Yout, in_pitch,
@@ -841,7 +836,7 @@ static cudaError_t launch_colfft_t(V* S, int ncols, int nouter, long long outer_
                                    cudaStream_t st, int nsim, long long sim_stride) {
     constexpr int TC = col_tile(L, 1, sizeof(V));
     const size_t smem = (size_t)TC * line_len(L) * sizeof(V);
-    cudaError_t e = set_smem(colfft_kernel<L, SIGN, V>, smem);
+    cudaError_t e = allow_smem(colfft_kernel<L, SIGN, V>, smem);
     if (e != cudaSuccess) return e;
     int ntiles = (ncols + TC - 1) / TC;
     int threads = TC * tpl(L);
@@ -860,7 +855,7 @@ static cudaError_t launch_colfft4_t(float2* S, int ncols, int nouter, long long 
     auto smem_of = [](int tc) { return (size_t)(tc * col4_stride<L>(tc) + F::TWT) * sizeof(float2); };
     if (TC < 1 || TC > 16 || TC * F::P2 > 512 || smem_of(TC) > 200 * 1024) TC = col4_tile(L);
     const size_t smem = smem_of(TC);
-    cudaError_t e = set_smem(colfft4_kernel<L, SIGN>, smem);
+    cudaError_t e = allow_smem(colfft4_kernel<L, SIGN>, smem);
     if (e != cudaSuccess) return e;
     const int ntiles = (ncols + TC - 1) / TC;
     int threads = TC * F::P2;
@@ -932,7 +927,7 @@ static cudaError_t launch_colmul4_s(float2* S, const KernelView& K, int ncols, i
     constexpr int TC = colmul4_tc<L, SHIFT>();
     const int cstride = col4_stride<L>(TC < 16 ? TC : 16) > F::LBUF ? col4_stride<L>(TC < 16 ? TC : 16) : F::LBUF;
     const size_t smem = (size_t)(3 * TC * cstride + F::TWT) * sizeof(float2);
-    cudaError_t e = set_smem(colmul4_kernel<L, TC, ZAX>, smem);
+    cudaError_t e = allow_smem(colmul4_kernel<L, TC, ZAX>, smem);
     if (e != cudaSuccess) return e;
     int threads = 3 * TC * F::P2;
     if (threads < 32) threads = 32;
@@ -950,7 +945,7 @@ static cudaError_t launch_colmul_split(float2* S, const KernelView& K, int ncols
                                        long long sim_stride, const float* sim_scale) {
     const int cstride = col4_stride<H>(TC);
     const size_t smem = (size_t)(3 * TC * cstride + FS<H>::TWT) * sizeof(float2);
-    cudaError_t e = set_smem(colmul_split_kernel<H, TC>, smem);
+    cudaError_t e = allow_smem(colmul_split_kernel<H, TC>, smem);
     if (e != cudaSuccess) return e;
     return launch_pdl(colmul_split_kernel<H, TC>, dim3((unsigned)((ncols + TC - 1) / TC), (unsigned)nsim),
                       dim3(3 * TC * FS<H>::P2), smem, st, S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl,

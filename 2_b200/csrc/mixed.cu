@@ -103,11 +103,6 @@ template <typename V> static bool table_of(int L, const V** out) {
     return true;
 }
 
-template <typename KT> static cudaError_t mr_smem(KT kern, size_t bytes) {
-    if (bytes > 48 * 1024) return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    return cudaSuccess;
-}
-
 // ---------------------------------------------------------------- R2C row pass
 // As xfwd_kernel: rows r = (c*Z + z)*Y + y of n_in reals (times the mask), zero-padded to
 // 2M, packed as z[e] = x[2e] + i x[2e+1], transformed (length M) and post-processed into
@@ -180,7 +175,7 @@ cudaError_t launch_mr_xfwd(int M, const S* in, PP pp, const float* mask, V* out,
     const int nt = mr_row_threads(M);
     const int rpb = 256 / nt;
     const size_t smem = (size_t)rpb * 2 * M * sizeof(V);
-    cudaError_t e = mr_smem(mr_xfwd_kernel<V, S>, smem);
+    cudaError_t e = allow_smem(mr_xfwd_kernel<V, S>, smem);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((nrows + rpb - 1) / rpb), (unsigned)nsim);
     mr_xfwd_kernel<V, S><<<grid, rpb * nt, smem, st>>>(in, pp, mask, out, nrows, Z, Y, Yout, in_pitch, n_in, hp, f,
@@ -253,7 +248,7 @@ cudaError_t launch_mr_xfwd<float2, float>(int M, const float* in, PP pp, const f
     P.sh = sh;
     P.pitch = (1 << sh) + 1;
     const size_t smem = lines_smem(M, 1 << sh);
-    cudaError_t e = mr_smem(mr_rows_kernel, smem);
+    cudaError_t e = allow_smem(mr_rows_kernel, smem);
     if (e != cudaSuccess) return e;
     const int tc = 1 << sh, threads = std::min(256, std::max(64, (tc * P.nq + 31) / 32 * 32));
     return launch_pdl(mr_rows_kernel, dim3((unsigned)((nrows + tc - 1) / tc), (unsigned)nsim), dim3(threads), smem, st,
@@ -318,11 +313,11 @@ cudaError_t launch_mr_colfft(int L, int sign, V* S, int ncols, int nouter, long 
     const dim3 grid((unsigned)(nouter * ntiles), (unsigned)nsim);
     cudaError_t e;
     if (sign < 0) {
-        if ((e = mr_smem(mr_colfft_kernel<-1, V>, smem)) != cudaSuccess) return e;
+        if ((e = allow_smem(mr_colfft_kernel<-1, V>, smem)) != cudaSuccess) return e;
         mr_colfft_kernel<-1, V><<<grid, 256, smem, st>>>(S, ncols, outer_stride, line_stride, n_in, n_out, f, tw, ctl,
                                                          skip_retry, sim_stride, TC);
     } else {
-        if ((e = mr_smem(mr_colfft_kernel<1, V>, smem)) != cudaSuccess) return e;
+        if ((e = allow_smem(mr_colfft_kernel<1, V>, smem)) != cudaSuccess) return e;
         mr_colfft_kernel<1, V><<<grid, 256, smem, st>>>(S, ncols, outer_stride, line_stride, n_in, n_out, f, tw, ctl,
                                                         skip_retry, sim_stride, TC);
     }

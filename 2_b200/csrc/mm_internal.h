@@ -301,6 +301,16 @@ bool epi_r2c_supported(int M);
 // into the spectrum S (times the Msat mask when fwd_mask), for M with epi_r2c_supported(M)
 cudaError_t launch_combine_rows(int M, const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
                                 long long spec_bstride, const float2* tw, int fwd_mask, int nsim, cudaStream_t st);
+// Lets launches of `kern` take `bytes` of dynamic shared memory.  The limit belongs to the
+// function, not to the launch: one set to each launch's own size would be lowered by a smaller
+// launch of another host thread between this call and the launch.  So every launch sets the
+// same value, the 227 KB that a block can have less 8 KB for the kernel's static arrays.
+constexpr size_t MM_SMEM_MOST = 219 * 1024;
+template <typename KT> inline cudaError_t allow_smem(KT kern, size_t bytes) {
+    if (bytes <= 48 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(bytes > MM_SMEM_MOST ? bytes : MM_SMEM_MOST));
+}
 int report_error(int code, const char* msg);  // sets mm_last_error()
 int local_blocks(long long N, int nsim = 1);
 

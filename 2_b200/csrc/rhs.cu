@@ -1007,11 +1007,8 @@ static cudaError_t launch_combine_rows_t(const CombineArgs& A, const int n[3], f
     const RowTile tile = xinv4_shape<M>(n[0] * n[1], n[2], nsim, 0);
     const int RPB = tile.rpb, threads = tile.threads;
     const size_t smem = (size_t)(RPB * 3 * FS<M>::LBUF + FS<M>::TWT + M / 2 + 1) * sizeof(float2);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(combine_rows_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(combine_rows_kernel<M>, smem);
+    if (e != cudaSuccess) return e;
     const int blocks = (n[0] * n[1] + RPB - 1) / RPB;
     return launch_pdl(combine_rows_kernel<M>, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, A, n[0],
                       n[1], n[2], S, hp, L1, spec_bstride, tw, fwd_mask, RPB);
@@ -1302,11 +1299,8 @@ static cudaError_t launch_xinv_t(const float2* S, int hp, int L1, const float2* 
     int rpb = (3 * TPL >= 384) ? 1 : 384 / (3 * TPL);
     size_t smem = (size_t)rpb * 3 * line_len(M) * sizeof(float2);
     while (smem > 100 * 1024 && rpb > 1) { rpb /= 2; smem = (size_t)rpb * 3 * line_len(M) * sizeof(float2); }
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(xinv_epi_kernel<M, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(xinv_epi_kernel<M, TERMS>, smem);
+    if (e != cudaSuccess) return e;
     const int nrows = A.P.n[0] * A.P.n[1];
     int blocks = (nrows + rpb - 1) / rpb;
     int threads = rpb * 3 * TPL;
@@ -1435,11 +1429,8 @@ static cudaError_t launch_mr_combine_rows(int M, const CombineArgs& A, const int
     mr_xinv_shape(M, n[0] * n[1], n[2], nsim, &rpb, &P.sh, &threads);
     P.pitch = (1 << P.sh) + 1;
     const size_t smem = lines_smem(M, 1 << P.sh);
-    if (smem > 48 * 1024) {
-        const cudaError_t e =
-            cudaFuncSetAttribute(mr_combine_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(mr_combine_rows_kernel, smem);
+    if (e != cudaSuccess) return e;
     const int blocks = (n[0] * n[1] + rpb - 1) / rpb;
     return launch_pdl(mr_combine_rows_kernel, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, A, n[0],
                       n[1], n[2], S, hp, L1, spec_bstride, P, twM, tw2M, fwd_mask, rpb);
@@ -1467,10 +1458,8 @@ static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, cons
         else if ((spec & NOMS) == NOMS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMS>;
         else if ((spec & NOMT) == NOMT) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMT>;
     }
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(kern, smem);
+    if (e != cudaSuccess) return e;
     const int nrows = A.P.n[0] * A.P.n[1];
     const int blocks = (nrows + rpb - 1) / rpb;
     *nblocks = blocks;
@@ -1507,10 +1496,8 @@ static cudaError_t launch_xinv4_h(const float2* S, int hp, int L1, const float2*
         if ((spec & NOTS) == NOTS) kern = xinv4_epi_kernel<M, false, FLEX, FWD, NOTS>;
         else if ((spec & NOMT) == NOMT) kern = xinv4_epi_kernel<M, false, FLEX, FWD, NOMT>;
     }
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = allow_smem(kern, smem);
+    if (e != cudaSuccess) return e;
     // batched plans: two blocks per SM (the launch bounds) need the shared-memory carveout
     // as well; single plans keep the default split, whose larger L1 serves the stencil's
     // neighbour loads

@@ -733,8 +733,7 @@ extern "C" MM_API int mm_nn_conv3x3_wgrad(const void* dy, int dy_cs, int dy_co, 
     // keep the kernel that stages each tap
     if (ring <= 1024 && total < (1LL << 30)) {
         const size_t smem = (size_t)(ring + 2 * WR_KC) * WR_PITCH * sizeof(bf16) + (size_t)ring * sizeof(int);
-        const cudaError_t e = cudaFuncSetAttribute(conv3x3_wgrad_ring_kernel,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        const cudaError_t e = allow_smem(conv3x3_wgrad_ring_kernel, smem);
         if (e != cudaSuccess) return report_error(MM_ERR_CUDA, cudaGetErrorString(e));
         // three blocks per SM, at least four stages each (a block starts with 2 (W + 2)
         // positions of halo and ends with 9216 reductions)
@@ -1144,8 +1143,7 @@ static cudaError_t launch_conv_tc_st(const bf16* in, int in_cs, int in_co, int C
                                      bf16* out, int out_cs, int out_co, int Cout, int B, int H, int Wd, int relu,
                                      int* err, cudaStream_t st, int band, int stage_bytes) {
     const int smem = ST * stage_bytes;
-    cudaError_t e =
-        cudaFuncSetAttribute(conv3x3_tc_kernel<N, ST, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(conv3x3_tc_kernel<N, ST, T>, smem);
     if (e != cudaSuccess) return e;
     const long long positions = (long long)B * (H + 1) * (Wd + 1);
     dim3 grid((unsigned)((positions + 128 * T - 1) / (128 * T)), (unsigned)((Cout + N - 1) / N));
@@ -1408,7 +1406,7 @@ static cudaError_t launch_conv_tcp_st(const bf16* in, int in_cs, int in_co, int 
                                       bf16* out, int out_cs, int out_co, int Cout, int B, int H, int Wd, int relu,
                                       int* err, cudaStream_t st, int band, int stage_bytes) {
     const int smem = ST * stage_bytes;
-    cudaError_t e = cudaFuncSetAttribute(conv3x3_tcp_kernel<N, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(conv3x3_tcp_kernel<N, ST>, smem);
     if (e != cudaSuccess) return e;
     const long long positions = (long long)B * (H + 1) * (Wd + 1);
     const int ntiles = (int)((positions + 127) / 128);
@@ -1656,8 +1654,7 @@ static cudaError_t launch_wgrad_tc_st(const bf16* dy, int dy_cs, int dy_co, int 
     // columns, four blocks fit the TMEM and shared memory is limited to a quarter
     const int smem = TG == 9 ? (ST * stage_bytes > 116 * 1024 ? ST * stage_bytes : 116 * 1024)
                              : (ST * stage_bytes > 56 * 1024 ? ST * stage_bytes : 56 * 1024);
-    cudaError_t e =
-        cudaFuncSetAttribute(conv3x3_wgrad_tc_kernel<ST, TG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaError_t e = allow_smem(conv3x3_wgrad_tc_kernel<ST, TG>, smem);
     if (e != cudaSuccess) return e;
     const long long total = (long long)B * (H + 1) * (Wd + 1);
     const int ct = (Cin + 31) / 32, mt = (Cout + 127) / 128;
