@@ -340,8 +340,8 @@ bool col_plan(int L, bool split, int cap, int cap_last, const float2* tw_pow2, C
     }
     for (int s = 0; s < P->nst; s++) P->r[s] = best[s];
     P->nq = P->N / P->r[P->nst - 1];
-    P->sh = 0;
-    P->pitch = 1;
+    P->big = best[0] > 10;  // descending order
+    set_lines(P, 1);
     if (mr_pow2(L)) {
         P->tws = TWN / L;
         *tw = tw_pow2;
@@ -360,7 +360,7 @@ cudaError_t launch_colmix_fft(int L, int sign, float2* S, int ncols, int nouter,
     const size_t line = (size_t)P.NP * P.N * sizeof(float2);
     const int tc = pick_cols(line, ncols, (long long)nouter * nsim);
     const size_t smem = line * tc;
-    P.sh = tc == 16 ? 4 : (tc == 8 ? 3 : (tc == 4 ? 2 : 1));
+    set_lines(&P, tc);
     P.pitch = tc;
     const int threads = pick_threads(P.NP * P.nq * tc);
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
@@ -383,7 +383,7 @@ cudaError_t launch_colmix_mul(int L, float2* S, const KernelView& K, int ncols, 
     if (tile < 0 && tc > 2) tc /= 2;
     if (tile > 0 && tc < 16 && line * tc * 2 <= 200 * 1024) tc *= 2;
     const size_t smem = line * tc;
-    P.sh = tc == 16 ? 4 : (tc == 8 ? 3 : (tc == 4 ? 2 : 1));
+    set_lines(&P, tc);
     P.pitch = tc;
     if (smem > 220 * 1024) return cudaErrorNotSupported;
     const int threads = pick_threads(std::max(P.NP * P.nq, 3 * P.N / P.r[0]) * tc);

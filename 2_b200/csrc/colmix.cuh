@@ -18,9 +18,18 @@ struct ColPlan {
     int r[MC_MAXST];  // radices in the order of the forward stages; the last one is the smallest
     int nq;           // N / r[nst - 1]
     int tws;          // W_L^m = tw[m * tws]
-    int sh;           // log2 of the lines per block (TC)
-    int pitch;        // shared-memory distance of a line's elements: TC, or TC + 1 where rows are transposed
+    int big;          // a radix above 10 (the row passes' run-time radix)
+    int tc;           // lines per block (TC)
+    int sh;           // log2 of TC where it is a power of two
+    unsigned rcp;     // 0 there, else ceil(2^32 / TC): element / TC without a division
+    int pitch;        // shared-memory distance of a line's elements: TC, odd where rows are transposed
 };
+
+// split(e): e = q * TC + line
+__device__ __forceinline__ int line_of(const ColPlan& P, int e, int& q) {
+    q = P.rcp ? (int)__umulhi((unsigned)e, P.rcp) : e >> P.sh;
+    return e - q * P.tc;
+}
 
 // a run-time radix 17..31 (prime): the paired sums of dft_prime on a local array, constants
 // from the twiddle table (W_R^m = tw[m * step])
@@ -87,7 +96,9 @@ __device__ __forceinline__ float2 tw_l(const ColPlan& P, const float2* __restric
         default: CALL(0); break;                                                                               \
     }
 
-// the row passes' radices: at most 10, which leaves the epilogue two blocks per SM
+// The row passes' radices: at most 10, and the run-time radix only in the kernels of lengths that
+// need it (BIG): its local array and body cost every other length registers and instruction
+// fetches.
 #define MC_SWITCH_ROW(rad, CALL)                                                                               \
     switch (rad) {                                                                                             \
         case 1: CALL(1); break;                                                                                \
@@ -100,18 +111,20 @@ __device__ __forceinline__ float2 tw_l(const ColPlan& P, const float2* __restric
         case 8: CALL(8); break;                                                                                \
         case 9: CALL(9); break;                                                                                \
         case 10: CALL(10); break;                                                                              \
-        default: CALL(0); break;                                                                               \
+        default:                                                                                               \
+            if constexpr (BIG) { CALL(0); }                                                                    \
+            break;                                                                                             \
     }
 
 // ---- a middle stage of sub-blocks of ncur elements (forward, or its mirror image)
 template <int R, int SIGN>
 __device__ __forceinline__ void mid_stage(const ColPlan& P, int rad, int ncur, float2* sm, int lines,
                                           const float2* __restrict__ tw) {
-    const int TC = 1 << P.sh;
-    const int M = ncur / rad, per = P.N / rad * TC, ts = P.N / ncur * P.NP;
+    const int M = ncur / rad, per = P.N / rad * P.tc, ts = P.N / ncur * P.NP;
     for (int i = threadIdx.x; i < lines * per; i += blockDim.x) {
-        const int l = i / per, e = i - l * per;
-        const int col = e & (TC - 1), q = e >> P.sh;
+        const int l = lines == 1 ? 0 : i / per;
+        int q;
+        const int col = line_of(P, i - l * per, q);
         const int blk = q / M, j = q - blk * M;
         float2* x = sm + (l * P.N + blk * ncur + j) * P.pitch + col;
         float2 v[RegLen<R>::n];
@@ -152,8 +165,10 @@ __device__ __forceinline__ int freq_slot(const ColPlan& P, int k) {
 
 // The whole transform of the block's TC lines in shared memory: forward (natural order in,
 // digit-reversed slots out) or its mirror image.  Synchronises the block after each stage.
-template <int SIGN>
-__device__ __noinline__ void lines_fft(const ColPlan& P, float2* sm, const float2* __restrict__ tw) {
+// Inlined: as a called function it made every epilogue spill 128-640 bytes at 80 registers, and
+// small grids wait for its instructions (256 rows of 192 cells, C2R + epilogue 18.1 -> 14.4 us).
+template <int SIGN, bool BIG>
+__device__ __forceinline__ void lines_fft(const ColPlan& P, float2* sm, const float2* __restrict__ tw) {
     int ncur = SIGN < 0 ? P.N : 1;
     for (int i = 0; i < P.nst; i++) {
         const int rad = P.r[SIGN < 0 ? i : P.nst - 1 - i];
@@ -172,12 +187,12 @@ __device__ __forceinline__ void fill_slots(const ColPlan& P, unsigned short* slo
 }
 
 // Real-to-complex post-processing of one transformed line (the packed sequence
-// x[2n] + i x[2n+1], element e at line[e * pitch]) by one warp: X[k] = E[k] + W_2M^k O[k],
-// k <= M, to dst.
+// x[2n] + i x[2n+1], element e at line[e * pitch]): X[k] = E[k] + W_2M^k O[k], k <= M, to dst,
+// for k0, k0 + kstep ... up to M / 2 and their mirror images.
 __device__ __forceinline__ void r2c_line(const ColPlan& P, const float2* line, const unsigned short* slot,
-                                         const float2* __restrict__ tw2M, int lane, float2* dst) {
+                                         const float2* __restrict__ tw2M, int k0, int kstep, float2* dst) {
     const int M = P.N;
-    for (int k = lane; k <= M / 2; k += 32) {
+    for (int k = k0; k <= M / 2; k += kstep) {
         const float2 zk = line[slot[k] * P.pitch];
         const float2 zm = line[slot[k ? M - k : 0] * P.pitch];
         const float2 e = make_float2(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y));
@@ -188,12 +203,12 @@ __device__ __forceinline__ void r2c_line(const ColPlan& P, const float2* line, c
     }
 }
 
-// Complex-to-real pre-processing of one spectrum row by one warp, into the slots that the
-// inverse starts from: Z[k] = (X[k] + conj X[M-k]) + i W_2M^-k (X[k] - conj X[M-k]).
+// Complex-to-real pre-processing of one spectrum row, into the slots that the inverse starts
+// from: Z[k] = (X[k] + conj X[M-k]) + i W_2M^-k (X[k] - conj X[M-k]), k = k0, k0 + kstep ... < M.
 __device__ __forceinline__ void c2r_line(const ColPlan& P, float2* line, const unsigned short* slot,
-                                         const float2* __restrict__ tw2M, int lane, const float2* src) {
+                                         const float2* __restrict__ tw2M, int k0, int kstep, const float2* src) {
     const int M = P.N;
-    for (int k = lane; k < M; k += 32) {
+    for (int k = k0; k < M; k += kstep) {
         const float2 a = src[k], b = src[M - k];
         const float2 s = make_float2(a.x + b.x, a.y - b.y);
         const float2 d = make_float2(a.x - b.x, a.y + b.y);
@@ -205,7 +220,15 @@ __device__ __forceinline__ void c2r_line(const ColPlan& P, float2* line, const u
 
 // shared memory of tc transposed lines of length M with their slot table
 inline size_t lines_smem(int M, int tc) {
-    return (size_t)M * (tc + 1) * sizeof(float2) + (size_t)(M + 3) / 4 * 4 * sizeof(unsigned short);
+    return (size_t)M * (tc | 1) * sizeof(float2) + (size_t)(M + 3) / 4 * 4 * sizeof(unsigned short);
+}
+// tc lines per block in the plan of a row pass; an odd pitch
+inline void set_lines(ColPlan* P, int tc) {
+    P->tc = tc;
+    P->sh = 0;
+    while (1 << P->sh < tc) P->sh++;
+    P->rcp = 1 << P->sh == tc ? 0u : (unsigned)((((unsigned long long)1 << 32) + tc - 1) / tc);
+    P->pitch = tc | 1;
 }
 
 // Host: the stages of length L (split: as two half-length transforms by parity, NP = 2) from

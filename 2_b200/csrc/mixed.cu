@@ -184,11 +184,21 @@ cudaError_t launch_mr_xfwd(int M, const S* in, PP pp, const float* mask, V* out,
     return cudaGetLastError();
 }
 
-// The FP32 row pass: TC rows per block side by side in shared memory (colmix.cuh), a warp per
-// row between global memory and the transposed lines (pitch TC + 1: consecutive elements of
+// Rows per block of the FP32 row pass: 16, fewer while the lines take more than 56 KB or leave
+// less than two blocks per SM, and one only to leave one block per SM (torque of 32 rows of 1500
+// cells 52.6 us with 4, 46.6 with 2, 44.1 with 1; of 256 rows 79.7, 74.3 and 82.7).
+static int rows_per_block(int M, long long rows) {
+    int tc = 16;
+    while (tc > 2 && ((tc > 4 && lines_smem(M, tc) > 56 * 1024) || rows / tc < 296)) tc /= 2;
+    return rows / tc < 148 ? 1 : tc;
+}
+
+// The FP32 row pass: TC rows per block side by side in shared memory (colmix.cuh), whole warps per
+// row between global memory and the transposed lines (an odd pitch: consecutive elements of
 // a row fall on distinct banks).  With the epilogue in the same form, 192x192x8 cells, RK12
 // step 253 -> 219 us; latency-bound.  Natural order through a second buffer instead of the slot
 // table took 1 % more (half the lines per SM).
+template <bool BIG>
 __global__ void __launch_bounds__(256, 3) mr_rows_kernel(const float* __restrict__ in_fixed, PP in_pp,
                                                          const float* __restrict__ mask, float2* __restrict__ out,
                                                          int nrows, int Z, int Y, int Yout, int in_pitch, int n_in,
@@ -204,18 +214,20 @@ __global__ void __launch_bounds__(256, 3) mr_rows_kernel(const float* __restrict
     const float* in = (in_fixed ? in_fixed : in_pp.get(ctl ? ctl->cur : 0)) + sim * in_bstride;
     out += sim * out_bstride;
     if (mask) mask += sim * mask_bstride;
-    const int M = P.N, TC = 1 << P.sh;
+    const int M = P.N, TC = P.tc;
     extern __shared__ unsigned char smem_raw[];
     float2* sm = reinterpret_cast<float2*>(smem_raw);
     unsigned short* slot = reinterpret_cast<unsigned short*>(sm + M * P.pitch);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     fill_slots(P, slot);
-    for (int l = warp; l < TC; l += nw) {
+    const int parts = max(1, nw / TC);  // warps per row
+    for (int w = warp; w < TC * parts; w += nw) {
+        const int l = w & (TC - 1), e0 = w / TC * 32 + lane;
         const int row = blockIdx.x * TC + l;
         const float* src = in + (long long)row * in_pitch;
         const float* msk = mask ? mask + (long long)(row % (Z * Y)) * in_pitch : nullptr;
         const int n = row < nrows ? n_in : 0;
-        for (int e = lane; e < M; e += 32) {
+        for (int e = e0; e < M; e += 32 * parts) {
             float2 v = make_float2(0.f, 0.f);
             if (2 * e < n) v.x = src[2 * e] * (msk ? msk[2 * e] : 1.f);
             if (2 * e + 1 < n) v.y = src[2 * e + 1] * (msk ? msk[2 * e + 1] : 1.f);
@@ -223,13 +235,14 @@ __global__ void __launch_bounds__(256, 3) mr_rows_kernel(const float* __restrict
         }
     }
     __syncthreads();
-    lines_fft<-1>(P, sm, twM);
-    for (int l = warp; l < TC; l += nw) {
+    lines_fft<-1, BIG>(P, sm, twM);
+    for (int w = warp; w < TC * parts; w += nw) {
+        const int l = w & (TC - 1), k0 = w / TC * 32 + lane;
         const int row = blockIdx.x * TC + l;
-        if (row >= nrows) break;
+        if (row >= nrows) continue;
         const int c = row / (Z * Y), zy = row - c * (Z * Y);
         const int z = zy / Y, y = zy - z * Y;
-        r2c_line(P, sm + l, slot, tw2M, lane, out + ((long long)(c * Z + z) * Yout + y) * hp);
+        r2c_line(P, sm + l, slot, tw2M, k0, 32 * parts, out + ((long long)(c * Z + z) * Yout + y) * hp);
     }
 }
 
@@ -241,17 +254,15 @@ cudaError_t launch_mr_xfwd<float2, float>(int M, const float* in, PP pp, const f
     ColPlan P;
     const float2 *twM = nullptr, *tw2M = nullptr;
     if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !table_of<float2>(2 * M, &tw2M)) return cudaErrorInvalidValue;
-    // 16 rows per block, fewer for long rows and for grids of less than two blocks per SM
-    int sh = 4;
-    while (sh > 2 && (lines_smem(M, 1 << sh) > 56 * 1024 || (long long)(nrows >> sh) * nsim < 296)) sh--;
-    while (sh > 0 && lines_smem(M, 1 << sh) > 200 * 1024) sh--;
-    P.sh = sh;
-    P.pitch = (1 << sh) + 1;
-    const size_t smem = lines_smem(M, 1 << sh);
-    cudaError_t e = allow_smem(mr_rows_kernel, smem);
+    const int tc = rows_per_block(M, (long long)nrows * nsim);
+    set_lines(&P, tc);
+    const size_t smem = lines_smem(M, tc);
+    const auto kern = P.big ? mr_rows_kernel<true> : mr_rows_kernel<false>;
+    const cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
-    const int tc = 1 << sh, threads = std::min(256, std::max(64, (tc * P.nq + 31) / 32 * 32));
-    return launch_pdl(mr_rows_kernel, dim3((unsigned)((nrows + tc - 1) / tc), (unsigned)nsim), dim3(threads), smem, st,
+    // a thread per element where the rows are few, else per radix of the last stage
+    const int threads = std::min(256, std::max(64, ((tc <= 2 ? tc * M : tc * P.nq) + 31) / 32 * 32));
+    return launch_pdl(kern, dim3((unsigned)((nrows + tc - 1) / tc), (unsigned)nsim), dim3(threads), smem, st,
                       in, pp, mask, out, nrows, Z, Y, Yout, in_pitch, n_in, hp, P, twM, tw2M, ctl, skip_retry,
                       in_bstride, out_bstride, mask_bstride);
 }

@@ -1310,37 +1310,44 @@ static cudaError_t launch_xinv_t(const float2* S, int hp, int L1, const float2* 
     return cudaGetLastError();
 }
 
+#endif  // MM_RHS_PART == 0
+
 // ---------------------------------------------------------------- mixed-radix C2R + epilogue
 // R2C rows from transposed lines whose float x (element x/2, part x mod 2) holds the input at
 // cell x < n2; line 3*lrow + c is row row0 + lrow of component c.  Called by the whole block.
+template <bool BIG>
 __device__ __forceinline__ void staged_rows_r2c(const ColPlan& P, float2* sm, const unsigned short* slot,
                                                 const float2* __restrict__ twM, const float2* __restrict__ tw2M,
                                                 int row0, int lines, int n0, int n1, int n2, float2* S, int hp,
                                                 int L1) {
-    const int TC = 1 << P.sh;
-    for (int i = threadIdx.x; i < (P.N - n2 / 2) * TC; i += blockDim.x) {
-        const int e = n2 / 2 + (i >> P.sh);
-        float2* q = sm + e * P.pitch + (i & (TC - 1));
+    for (int i = threadIdx.x; i < (P.N - n2 / 2) * P.tc; i += blockDim.x) {
+        int e;
+        const int l = line_of(P, i, e);
+        e += n2 / 2;
+        float2* q = sm + e * P.pitch + l;
         if (2 * e < n2) q->y = 0.f;
         else *q = make_float2(0.f, 0.f);
     }
     __syncthreads();
-    lines_fft<-1>(P, sm, twM);
+    lines_fft<-1, BIG>(P, sm, twM);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int l = warp; l < lines; l += nw) {
+    const int parts = max(1, nw / lines);  // warps per line
+    for (int w = warp; w < lines * parts; w += nw) {
+        const int part = w / lines, l = w - part * lines;
         const int row = row0 + l / 3, c = l % 3;
         const int z = row / n1, y = row - z * n1;
-        r2c_line(P, sm + l, slot, tw2M, lane, S + ((long long)(c * n0 + z) * L1 + y) * hp);
+        r2c_line(P, sm + l, slot, tw2M, part * 32 + lane, 32 * parts, S + ((long long)(c * n0 + z) * L1 + y) * hp);
     }
 }
 
 // Row lengths M that are not powers of two: rpb rows of three component lines side by side
-// in shared memory (colmix.cuh), a warp per spectrum row for the pre-processing, the in-place
+// in shared memory (colmix.cuh), whole warps per spectrum row for the pre-processing, the in-place
 // inverse, then the same epilogue.  BATCH: the simulation's scalars are staged in shared
 // memory (batched plans, time tables).
 // FWD: then the R2C rows of the next stage state into the spectrum rows just read, as
-// mr_rows_kernel makes them.
-template <bool TERMS, bool BATCH, bool FWD, int SPEC>
+// mr_rows_kernel makes them.  BIG: see MC_SWITCH_ROW.  64-80 registers (no spills) and two
+// blocks per SM; small grids are bound by instruction fetches (256 rows of 192 cells, 14.4 us).
+template <bool TERMS, bool BATCH, bool FWD, int SPEC, bool BIG>
 __global__ void __launch_bounds__(384, 2) mr_xinv_epi_kernel(typename SpecIn<FWD>::type S, int hp, int L1,
                                                           const __grid_constant__ ColPlan P,
                                                           const float2* __restrict__ twM,
@@ -1361,22 +1368,25 @@ __global__ void __launch_bounds__(384, 2) mr_xinv_epi_kernel(typename SpecIn<FWD
     fill_slots(P, slot);
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int l = warp; l < 3 * here; l += nw) {
+    const int lines = 3 * here, parts = max(1, nw / lines);  // warps per line
+    for (int w = warp; w < lines * parts; w += nw) {
+        const int part = w / lines, l = w - part * lines;
         const int row = row0 + l / 3, c = l % 3;
         const int z = row / n1, y = row - z * n1;
-        c2r_line(P, sm + l, slot, tw2M, lane, S + ((long long)(c * n0 + z) * L1 + y) * hp);
+        c2r_line(P, sm + l, slot, tw2M, part * 32 + lane, 32 * parts, S + ((long long)(c * n0 + z) * L1 + y) * hp);
     }
     __syncthreads();
-    lines_fft<+1>(P, sm, twM);
+    lines_fft<+1, BIG>(P, sm, twM);
     epilogue_rows<TERMS, false, BATCH, FWD, SPEC, true>(A, pick_scalars<BATCH>(s_sim, A.P.s), sm, P.pitch, row0, here);
     if constexpr (FWD) {
         __syncthreads();
-        staged_rows_r2c(P, sm, slot, twM, tw2M, row0, 3 * here, n0, n1, A.P.n[2],
-                        A.fwd + blockIdx.y * A.spec_bstride, hp, L1);
+        staged_rows_r2c<BIG>(P, sm, slot, twM, tw2M, row0, lines, n0, n1, A.P.n[2],
+                             A.fwd + blockIdx.y * A.spec_bstride, hp, L1);
     }
 }
 
 // combine_rows_kernel for these row lengths: the attempt's first stage state and its R2C rows.
+template <bool BIG>
 __global__ void __launch_bounds__(384, 2) mr_combine_rows_kernel(CombineArgs A, int n0, int n1, int n2, float2* S,
                                                                  int hp, int L1, long long spec_bstride,
                                                                  const __grid_constant__ ColPlan P,
@@ -1403,22 +1413,20 @@ __global__ void __launch_bounds__(384, 2) mr_combine_rows_kernel(CombineArgs A, 
         q[4] = nx.z * fm;
     }
     __syncthreads();
-    staged_rows_r2c(P, sm, slot, twM, tw2M, row0, 3 * here, n0, n1, n2, S + blockIdx.y * spec_bstride, hp, L1);
+    staged_rows_r2c<BIG>(P, sm, slot, twM, tw2M, row0, 3 * here, n0, n1, n2, S + blockIdx.y * spec_bstride, hp, L1);
 }
 
-// Rows per block (5, 2 or 1: three lines each of 16, 8 or 4) and threads of the mixed-radix
-// epilogue: 16 lines while they fit 56 KB and leave two blocks per SM.
-static void mr_xinv_shape(int M, int n0n1, int n2, int nsim, int* rpb, int* sh, int* threads) {
-    *sh = 4;
+// Rows per block (three lines each) and threads of the mixed-radix epilogue: five rows while
+// they fit 56 KB and leave two blocks per SM, else two or one.
+static void mr_xinv_shape(int M, int n0n1, int n2, int nsim, int* rpb, int* threads) {
     *rpb = 5;
-    while (*sh > 2 && (lines_smem(M, 1 << *sh) > 56 * 1024 || (long long)((n0n1 + *rpb - 1) / *rpb) * nsim < 296)) {
-        (*sh)--;
-        *rpb = (1 << *sh) / 3;
-    }
+    while (*rpb > 1 && (lines_smem(M, 3 * *rpb) > 56 * 1024 || (long long)((n0n1 + *rpb - 1) / *rpb) * nsim < 296))
+        *rpb /= 2;
     const int cells = *rpb * n2, turns = (cells + 383) / 384;
     *threads = std::max(96, ((cells + turns - 1) / turns + 31) / 32 * 32);
 }
 
+#if MM_RHS_PART == 0
 static cudaError_t launch_mr_combine_rows(int M, const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
                                           long long spec_bstride, int fwd_mask, int nsim, cudaStream_t st) {
     ColPlan P;
@@ -1426,37 +1434,36 @@ static cudaError_t launch_mr_combine_rows(int M, const CombineArgs& A, const int
     if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !mr_tables(2 * M, &tw2M, nullptr))
         return cudaErrorInvalidValue;
     int rpb, threads;
-    mr_xinv_shape(M, n[0] * n[1], n[2], nsim, &rpb, &P.sh, &threads);
-    P.pitch = (1 << P.sh) + 1;
-    const size_t smem = lines_smem(M, 1 << P.sh);
-    const cudaError_t e = allow_smem(mr_combine_rows_kernel, smem);
+    mr_xinv_shape(M, n[0] * n[1], n[2], nsim, &rpb, &threads);
+    set_lines(&P, 3 * rpb);
+    const size_t smem = lines_smem(M, P.tc);
+    const auto kern = P.big ? mr_combine_rows_kernel<true> : mr_combine_rows_kernel<false>;
+    const cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
     const int blocks = (n[0] * n[1] + rpb - 1) / rpb;
-    return launch_pdl(mr_combine_rows_kernel, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, A, n[0],
-                      n[1], n[2], S, hp, L1, spec_bstride, P, twM, tw2M, fwd_mask, rpb);
+    return launch_pdl(kern, dim3((unsigned)blocks, (unsigned)nsim), dim3(threads), smem, st, A, n[0], n[1], n[2], S, hp,
+                      L1, spec_bstride, P, twM, tw2M, fwd_mask, rpb);
 }
+#endif  // MM_RHS_PART == 0
 
-template <bool TERMS, bool BATCH, bool FWD>
-static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, const EpiArgs& A, cudaStream_t st,
-                                    int* nblocks, int nsim) {
-    ColPlan P;
-    const float2 *twM = nullptr, *tw2M = nullptr;
-    if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !mr_tables(2 * M, &tw2M, nullptr))
-        return cudaErrorInvalidValue;
+#if MM_RHS_PART >= 6
+template <bool TERMS, bool BATCH, bool FWD, bool BIG>
+static cudaError_t launch_mr_xinv_t(ColPlan& P, const float2* twM, const float2* tw2M, const float2* S, int hp, int L1,
+                                    const EpiArgs& A, cudaStream_t st, int* nblocks, int nsim) {
     int rpb, threads;
-    mr_xinv_shape(M, A.P.n[0] * A.P.n[1], A.P.n[2], nsim, &rpb, &P.sh, &threads);
-    P.pitch = (1 << P.sh) + 1;
-    const size_t smem = lines_smem(M, 1 << P.sh);
+    mr_xinv_shape(P.N, A.P.n[0] * A.P.n[1], A.P.n[2], nsim, &rpb, &threads);
+    set_lines(&P, 3 * rpb);
+    const size_t smem = lines_smem(P.N, P.tc);
     // the epilogue without what the evaluation lacks (as the four-step pass chooses it)
-    auto kern = mr_xinv_epi_kernel<TERMS, BATCH, FWD, 0>;
+    auto kern = mr_xinv_epi_kernel<TERMS, BATCH, FWD, 0, BIG>;
     if constexpr (!TERMS) {
         const int spec = epilogue_spec(A.P);
         constexpr int NOTS = SPEC_NOTHERMAL | SPEC_NOSTT, NOMS = SPEC_NOMASK | SPEC_NOSTT,
                       NOMT = SPEC_NOMASK | SPEC_NOTHERMAL;
-        if (spec == SPEC_LEAN) kern = mr_xinv_epi_kernel<false, BATCH, FWD, SPEC_LEAN>;
-        else if ((spec & NOTS) == NOTS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOTS>;
-        else if ((spec & NOMS) == NOMS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMS>;
-        else if ((spec & NOMT) == NOMT) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMT>;
+        if (spec == SPEC_LEAN) kern = mr_xinv_epi_kernel<false, BATCH, FWD, SPEC_LEAN, BIG>;
+        else if ((spec & NOTS) == NOTS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOTS, BIG>;
+        else if ((spec & NOMS) == NOMS) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMS, BIG>;
+        else if ((spec & NOMT) == NOMT) kern = mr_xinv_epi_kernel<false, BATCH, FWD, NOMT, BIG>;
     }
     const cudaError_t e = allow_smem(kern, smem);
     if (e != cudaSuccess) return e;
@@ -1467,7 +1474,30 @@ static cudaError_t launch_mr_xinv_t(int M, const float2* S, int hp, int L1, cons
                       rpb);
 }
 
-#endif  // MM_RHS_PART == 0
+#endif
+// The pass with or without per-term outputs, staged scalars and the next stage's rows.  The
+// instances of either BIG are a translation unit of their own (MM_RHS_PART, see build.py).
+template <bool BIG>
+cudaError_t launch_mr_xinv(ColPlan& P, const float2* twM, const float2* tw2M, const float2* S, int hp, int L1,
+                           const EpiArgs& A, bool terms, bool staged, cudaStream_t st, int* nblocks, int nsim)
+#if MM_RHS_PART >= 6
+{
+    if (terms) {
+        if (A.fwd) return cudaErrorInvalidValue;
+        return staged ? launch_mr_xinv_t<true, true, false, BIG>(P, twM, tw2M, S, hp, L1, A, st, nblocks, nsim)
+                      : launch_mr_xinv_t<true, false, false, BIG>(P, twM, tw2M, S, hp, L1, A, st, nblocks, 1);
+    }
+    if (A.fwd)
+        return staged ? launch_mr_xinv_t<false, true, true, BIG>(P, twM, tw2M, S, hp, L1, A, st, nblocks, nsim)
+                      : launch_mr_xinv_t<false, false, true, BIG>(P, twM, tw2M, S, hp, L1, A, st, nblocks, 1);
+    return staged ? launch_mr_xinv_t<false, true, false, BIG>(P, twM, tw2M, S, hp, L1, A, st, nblocks, nsim)
+                  : launch_mr_xinv_t<false, false, false, BIG>(P, twM, tw2M, S, hp, L1, A, st, nblocks, 1);
+}
+template cudaError_t launch_mr_xinv<MM_RHS_PART == 7>(ColPlan&, const float2*, const float2*, const float2*, int, int,
+                                                      const EpiArgs&, bool, bool, cudaStream_t, int*, int);
+#else
+;
+#endif
 
 template <int M, bool TERMS, bool BATCH, bool FLEX, bool FWD>
 static cudaError_t launch_xinv4_h(const float2* S, int hp, int L1, const float2* tw, const EpiArgs& A,
@@ -1539,7 +1569,7 @@ static cudaError_t launch_xinv4_t(const float2* S, int hp, int L1, const float2*
 template <int M>
 cudaError_t launch_xinv4(const float2* S, int hp, int L1, const float2* tw, const EpiArgs& A, bool terms, bool staged,
                          cudaStream_t st, int* nblocks, int nsim, int tile)
-#if MM_RHS_PART > 0
+#if MM_RHS_PART > 0 && MM_RHS_PART < 6
 {
     if (staged)
         return terms ? launch_xinv4_t<M, true, true>(S, hp, L1, tw, A, st, nblocks, nsim, tile)
@@ -1564,7 +1594,9 @@ X(1024)
 #undef X
 #else
 ;
+#endif
 
+#if MM_RHS_PART == 0
 static bool use_xinv4(int M) { return M >= 4 && M <= 1024 && mr_pow2(M); }
 
 // The row lengths whose epilogue can write the next stage's R2C rows: the four-step one and
@@ -1596,17 +1628,12 @@ cudaError_t launch_xinv_epi(int M, const float2* S, int hp, int L1, const float2
         }
     }
     if (!mr_pow2(M)) {  // not a power of two: the mixed-radix pass
-        const int ns = staged ? nsim : 1;
-        if (terms) {
-            if (A.fwd) return cudaErrorInvalidValue;
-            return staged ? launch_mr_xinv_t<true, true, false>(M, S, hp, L1, A, st, nblocks, ns)
-                          : launch_mr_xinv_t<true, false, false>(M, S, hp, L1, A, st, nblocks, ns);
-        }
-        if (A.fwd)
-            return staged ? launch_mr_xinv_t<false, true, true>(M, S, hp, L1, A, st, nblocks, ns)
-                          : launch_mr_xinv_t<false, false, true>(M, S, hp, L1, A, st, nblocks, ns);
-        return staged ? launch_mr_xinv_t<false, true, false>(M, S, hp, L1, A, st, nblocks, ns)
-                      : launch_mr_xinv_t<false, false, false>(M, S, hp, L1, A, st, nblocks, ns);
+        ColPlan P;
+        const float2 *twM = nullptr, *tw2M = nullptr;
+        if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !mr_tables(2 * M, &tw2M, nullptr))
+            return cudaErrorInvalidValue;
+        return P.big ? launch_mr_xinv<true>(P, twM, tw2M, S, hp, L1, A, terms, staged, st, nblocks, nsim)
+                     : launch_mr_xinv<false>(P, twM, tw2M, S, hp, L1, A, terms, staged, st, nblocks, nsim);
     }
     if (staged) return cudaErrorNotSupported;  // batched plans and time tables use the four-step pass
     switch (M) {
@@ -1642,6 +1669,6 @@ cudaError_t launch_local_epi(const EpiArgs& A, bool terms, cudaStream_t st, int*
     }
     return cudaGetLastError();
 }
-#endif  // MM_RHS_PART
+#endif  // MM_RHS_PART == 0
 
 }  // namespace mm
