@@ -12,7 +12,7 @@ OUT = os.path.join(HERE, "libmm_b200.so")
 SOURCES = ["conv.cu", "colmix.cu", "mixed.cu", "rhs.cu:5", "rhs.cu:7", "rhs.cu:6", "rhs.cu:4", "rhs.cu:3", "rhs.cu:2", "rhs.cu:1", "rhs.cu:0", "demag_setup.cu", "plan.cu", "compat.cu", "noalloc.cu", "io.cpp", "am12.cu", "unet.cu"]
 # "name:k" compiles name with -DMM_RHS_PART=k: the epilogue's instances in parts, in parallel
 # (eight cores: 12 min of compiling in 120 s)
-HEADERS = ["fft.cuh", "fft4.cuh", "mixed.cuh", "rdft.cuh", "colmix.cuh", "kernel_view.cuh", "pdl.cuh", "mm_internal.h"]
+HEADERS = ["fft.cuh", "fft4.cuh", "mixed.cuh", "rdft.cuh", "colmix.cuh", "tiles.h", "kernel_view.cuh", "pdl.cuh", "mm_internal.h"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden", "--diag-suppress", "177"]

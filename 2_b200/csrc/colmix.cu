@@ -21,6 +21,7 @@
 #include "kernel_view.cuh"
 #include "mm_internal.h"
 #include "pdl.cuh"
+#include "tiles.h"
 
 namespace mm {
 using namespace mmfft;
@@ -202,10 +203,11 @@ __device__ __forceinline__ void mid_stages(const ColPlan& P, float2* sm, int lin
 }
 
 // One component per line; block: outer index o, tile of TC columns.  192x192x8 cells (N = 192
-// in stages of 16 and 12): forward 32 -> 22 us, inverse 35 -> 26 (42 MB each); bound by the
-// twiddle loads and arithmetic of two blocks of 256 threads per SM (128 registers).
+// in stages of 16 and 12): forward 32 -> 22 us, inverse 35 -> 26 (21 MB each); bound by the
+// twiddle loads and arithmetic of two blocks of 256 threads per SM (128 registers, which also
+// lets one block have 512).
 template <int SIGN>
-__global__ void __launch_bounds__(256, 2) colmix_fft_kernel(float2* __restrict__ S, int ncols, long long outer_stride,
+__global__ void __launch_bounds__(512) colmix_fft_kernel(float2* __restrict__ S, int ncols, long long outer_stride,
                                                          long long ls, int n_in, int n_out, const __grid_constant__ ColPlan P,
                                                          const float2* __restrict__ tw, const DevCtl* ctl,
                                                          int skip_retry, long long sim_stride) {
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(256, 2) colmix_fft_kernel(float2* __restrict__
 // Three components per column: forward, symmetric kernel multiply, inverse.  kaxis 0: lines
 // along z (ky = o), 1: along y (kz = 0).  Bound by registers and shared memory (few warps);
 // lengths that are powers of two have faster four-step passes (conv.cu).
-__global__ void __launch_bounds__(256, 2) colmix_mul_kernel(float2* __restrict__ S, KernelView K, int ncols,
+__global__ void __launch_bounds__(512) colmix_mul_kernel(float2* __restrict__ S, KernelView K, int ncols,
                                                          long long comp_stride, long long outer_stride, long long ls,
                                                          int n_in, int kaxis, float scale, const __grid_constant__ ColPlan P,
                                                          const float2* __restrict__ tw, const DevCtl* ctl,
@@ -301,17 +303,7 @@ bool radix_search(int n, int left, int most, int cap, int* out, int depth, int* 
     return false;
 }
 
-// Columns per block: 16 (128-byte rows) while the lines fit 48 KB, fewer for longer lines
-// (2 at most 200 KB) and for grids of less than one block per SM.
-int pick_cols(size_t line_bytes, int ncols, long long outer) {
-    int tc = 16;
-    while (tc > 4 && line_bytes * tc > 50 * 1024) tc /= 2;
-    while (tc > 2 && line_bytes * tc > 200 * 1024) tc /= 2;
-    while (tc > 4 && (ncols + tc - 1) / tc * outer < 148) tc /= 2;
-    return tc;
-}
-
-int pick_threads(int work) { return std::min(256, std::max(64, (work + 31) / 32 * 32)); }
+int pick_threads(int work, int most) { return std::min(most, std::max(64, (work + 31) / 32 * 32)); }
 
 }  // namespace
 
@@ -358,11 +350,12 @@ cudaError_t launch_colmix_fft(int L, int sign, float2* S, int ncols, int nouter,
     const float2* tw = nullptr;
     if (!col_plan(L, L % 2 == 0 && 2 * std::min(n_in, n_out) <= L, 16, 16, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
     const size_t line = (size_t)P.NP * P.N * sizeof(float2);
-    const int tc = pick_cols(line, ncols, (long long)nouter * nsim);
+    const ColTile tile = col_tiles(line, ncols, (long long)nouter * nsim);
+    const int tc = tile.tc;
     const size_t smem = line * tc;
     set_lines(&P, tc);
     P.pitch = tc;
-    const int threads = pick_threads(P.NP * P.nq * tc);
+    const int threads = pick_threads(P.NP * P.nq * tc, tile.threads);
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
     cudaError_t e;
     auto kern = sign < 0 ? colmix_fft_kernel<-1> : colmix_fft_kernel<1>;
@@ -379,14 +372,15 @@ cudaError_t launch_colmix_mul(int L, float2* S, const KernelView& K, int ncols, 
     const float2* tw = nullptr;
     if (!col_plan(L, L % 2 == 0 && 2 * n_in <= L, 16, 8, tw_pow2, &P, &tw)) return cudaErrorInvalidValue;
     const size_t line = (size_t)3 * P.NP * P.N * sizeof(float2);
-    int tc = pick_cols(line, ncols, (long long)nouter * nsim);
-    if (tile < 0 && tc > 2) tc /= 2;
+    const ColTile shape = col_tiles(line, ncols, (long long)nouter * nsim);
+    int tc = shape.tc;
+    if (tile < 0 && tc > 1) tc /= 2;
     if (tile > 0 && tc < 16 && line * tc * 2 <= 200 * 1024) tc *= 2;
     const size_t smem = line * tc;
     set_lines(&P, tc);
     P.pitch = tc;
     if (smem > 220 * 1024) return cudaErrorNotSupported;
-    const int threads = pick_threads(std::max(P.NP * P.nq, 3 * P.N / P.r[0]) * tc);
+    const int threads = pick_threads(std::max(P.NP * P.nq, 3 * P.N / P.r[0]) * tc, shape.threads);
     const dim3 grid((unsigned)(nouter * ((ncols + tc - 1) / tc)), (unsigned)nsim);
     cudaError_t e;
     if ((e = allow_smem(colmix_mul_kernel, smem)) != cudaSuccess) return e;

@@ -27,6 +27,7 @@
 #include "mixed.cuh"
 #include "pdl.cuh"
 #include "rdft.cuh"
+#include "tiles.h"
 
 namespace mm {
 using namespace mmfft;
@@ -691,9 +692,10 @@ __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, Ke
 // exchange buffers at 2H: by the parity of the frequency, X[2k] = DFT_H(x)[k] and
 // X[2k+1] = DFT_H(x W_2H^n)[k], one after the other; the inverse's first H rows are the sum of
 // the two inverses, the odd one times W_2H^-n, kept in registers.  The input is read twice (the
-// second time from L2) and written at the end.  Four columns (32-byte rows) and 101 KB per
-// block, one block per SM by its registers; bound by the barriers between its phases with 12
-// warps: 91 us for 1024x1024 cells, where all 2048 frequencies at once took 156.
+// second time from L2) and written at the end.  Four columns (32-byte rows), 107 KB and 168
+// registers (a cap that spills 280 bytes) per thread of a block, one block per SM by its registers;
+// bound by the barriers between its phases with 12 warps: 91 us for 1024x1024 cells, where all
+// 2048 frequencies at once took 156.  Two columns on narrow films (split_columns).
 template <int H, int TC>
 __global__ void __launch_bounds__(3 * TC * FS<H>::P2, 1) colmul_split_kernel(
     float2* __restrict__ S, KernelView K, int ncols, long long comp_stride, long long line_stride, int n_in, float scale,
@@ -999,9 +1001,13 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
             default: break;
         }
     }
-    if (kaxis == 1 && nouter == 1 && L == 2048 && 2 * n_in <= L)
+    if (kaxis == 1 && nouter == 1 && L == 2048 && 2 * n_in <= L) {
+        if (split_columns(ncols, nsim) == 2)
+            return launch_colmul_split<1024, 2>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry,
+                                                st, nsim, sim_stride, sim_scale);
         return launch_colmul_split<1024, 4>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st,
                                             nsim, sim_stride, sim_scale);
+    }
     return launch_colmix_mul(L, S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, kaxis, scale, tw,
                              ctl, skip_retry, st, nsim, sim_stride, sim_scale, tile);
 }

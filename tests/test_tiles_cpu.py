@@ -1,0 +1,42 @@
+"""The host rules of csrc/tiles.h, compiled on their own (no GPU)."""
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "2_b200", "csrc")
+
+
+@pytest.fixture(scope="module")
+def rule(tmp_path_factory):
+    """rule(expression): the integer value of a C++ expression over tiles.h."""
+    d = tmp_path_factory.mktemp("tiles")
+
+    def run(*expr):
+        src = d / "t.cpp"
+        src.write_text('#include <cstdio>\n#include "tiles.h"\nusing namespace mm;\nint main() {\n'
+                       + "".join('std::printf("%%lld\\n", (long long)(%s));\n' % e for e in expr) + "}\n")
+        subprocess.run(["g++", "-std=c++17", "-Wall", "-Werror", "-I", CSRC, str(src), "-o", str(d / "t")], check=True)
+        return [int(v) for v in subprocess.run([str(d / "t")], check=True, capture_output=True, text=True).stdout.split()]
+    return run
+
+
+def test_columns_use_the_sms_of_narrow_films(rule):
+    """Narrow films take at least 60 blocks where they have the columns, and never more than one
+    block per SM by halving below four columns; wide ones keep rows of 32 bytes."""
+    line = {n1: 3 * 2 * n1 * 8 for n1 in (600, 1000, 1200, 2048)}
+    got = rule(*["col_tiles(%d, %d, 1).tc" % (line[n1], cols) for n1 in line for cols in (65, 129, 257, 1025)])
+    assert got == [1, 1, 2, 4, 1, 1, 2, 4, 1, 1, 2, 2, 1, 1, 2, 2]
+    # short lines keep four columns; the tile never passes 200 KB
+    assert rule("col_tiles(1536, 25, 6).tc", "col_tiles(98304, 65, 64).tc") == [4, 2]
+
+
+def test_column_threads(rule):
+    """512 where a block has its SM to itself."""
+    assert rule("col_tiles(28800, 1025, 1).threads", "col_tiles(30720, 1025, 1).threads",
+                "col_tiles(28800, 513, 1).threads", "col_tiles(1536, 97, 24).threads") == [256, 512, 512, 256]
+
+
+def test_split_columns(rule):
+    assert rule("split_columns(65, 1)", "split_columns(257, 1)", "split_columns(513, 1)", "split_columns(65, 8)") == \
+        [2, 2, 4, 4]
