@@ -1,4 +1,4 @@
-// tiles.h -- rules that choose the tiles of the column passes.  Plain C++ on the host, so that
+// tiles.h -- rules that choose tiles and kernels by the sizes of a launch.  Plain C++ on the host, so that
 // they can be checked without a GPU.
 #pragma once
 #include <algorithm>
@@ -37,5 +37,13 @@ inline ColTile col_tiles(size_t line_bytes, int ncols, long long outer) {
 // (1024 rows of 64 cells 155 -> 126 us a step, of 256 cells 214 -> 186; of 512 cells, 257 blocks
 // of 2: 257 -> 305).
 inline int split_columns(int ncols, int nsim) { return (long long)((ncols + 1) / 2) * nsim <= SMS ? 2 : 4; }
+
+// Which kernel sums a convolution's weight gradient, for `stages` of 64 positions and `tiles` of
+// 32 x 32 channels: the ring of positions, or the one that stages each tap.  The ring takes 7 us
+// however small the sum (its halo, one stage after the other, 9216 reductions a block); the
+// other's time grows with stages x (tiles + 3).  32x32 channels, the other and the ring: 4.4 and
+// 7.3 us (5 stages), 7.0 and 7.5 (162), 11.0 and 8.4 (324); 64x128, 81 stages: 9.6 and 9.3;
+// 256x256, 9: 8.7 and 8.5.
+inline bool wgrad_by_ring(long long stages, int tiles) { return stages * (tiles + 3) > 656; }
 
 }  // namespace mm

@@ -20,6 +20,7 @@
 #include <cstring>
 
 #include "mm_internal.h"
+#include "tiles.h"
 
 namespace mm {
 
@@ -729,19 +730,19 @@ extern "C" MM_API int mm_nn_conv3x3_wgrad(const void* dy, int dy_cs, int dy_co, 
     const long long total = (long long)B * (H + 1) * (Wd + 1);
     int ring = 256;
     while (ring < 3 * WR_KC + 2 * (Wd + 2)) ring *= 2;
-    // rows of up to 414 pixels (a ring of 1024 positions, two blocks per SM); longer ones
-    // keep the kernel that stages each tap
-    if (ring <= 1024 && total < (1LL << 30)) {
+    const long long stages = (total + WR_KC - 1) / WR_KC;
+    const int rmt = (Cout + 31) / 32, rnt = (Cin + 31) / 32;
+    // rows of up to 414 pixels (a ring of 1024 positions, two blocks per SM); longer ones and
+    // small sums keep the kernel that stages each tap
+    if (ring <= 1024 && total < (1LL << 30) && wgrad_by_ring(stages, rmt * rnt)) {
         const size_t smem = (size_t)(ring + 2 * WR_KC) * WR_PITCH * sizeof(bf16) + (size_t)ring * sizeof(int);
         const cudaError_t e = allow_smem(conv3x3_wgrad_ring_kernel, smem);
         if (e != cudaSuccess) return report_error(MM_ERR_CUDA, cudaGetErrorString(e));
         // three blocks per SM, at least four stages each (a block starts with 2 (W + 2)
         // positions of halo and ends with 9216 reductions)
-        const int mt = (Cout + 31) / 32, nt = (Cin + 31) / 32;
-        const long long stages = (total + WR_KC - 1) / WR_KC;
-        long long per = (stages * mt * nt + 148 * 3 - 1) / (148 * 3);
+        long long per = (stages * rmt * rnt + 148 * 3 - 1) / (148 * 3);
         per = std::min(stages, std::max(per, 4LL));
-        conv3x3_wgrad_ring_kernel<<<dim3((unsigned)mt, (unsigned)nt, (unsigned)((stages + per - 1) / per)), WR_THREADS,
+        conv3x3_wgrad_ring_kernel<<<dim3((unsigned)rmt, (unsigned)rnt, (unsigned)((stages + per - 1) / per)), WR_THREADS,
                                     smem, (cudaStream_t)st>>>(
             (const bf16*)dy, dy_cs, dy_co, Cout, (const bf16*)x, x_cs, x_co, Cin, dW, (int)total, (H + 1) * (Wd + 1), H,
             Wd, ring, (int)per * WR_KC, (reinterpret_cast<uintptr_t>(dW) & 7) == 0);

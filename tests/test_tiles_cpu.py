@@ -40,3 +40,10 @@ def test_column_threads(rule):
 def test_split_columns(rule):
     assert rule("split_columns(65, 1)", "split_columns(257, 1)", "split_columns(513, 1)", "split_columns(65, 8)") == \
         [2, 2, 4, 4]
+
+
+def test_small_weight_gradients_stage_each_tap(rule):
+    small = [(1, 1), (5, 1), (81, 1), (162, 1), (81, 4), (18, 16), (10, 48), (9, 48)]
+    large = [(289, 1), (133, 3), (81, 12), (67, 16), (21, 48), (4225, 64)]
+    assert rule(*["wgrad_by_ring(%d, %d)" % v for v in small]) == [0] * len(small)
+    assert rule(*["wgrad_by_ring(%d, %d)" % v for v in large]) == [1] * len(large)
