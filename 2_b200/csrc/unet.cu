@@ -503,8 +503,10 @@ __global__ void relu_bwd_kernel(const bf16* out, int o_cs, int o_co, bf16* d, in
 // of a pixel (16-byte loads; consecutive threads cover consecutive channels, then the
 // next pixels), zeroes the gradient where the forward output was not positive (relu),
 // keeps 8 register sums for its channels, and the block adds its per-channel sums to db.
-// Latency-bound on its loads: four pixels of a thread are in flight at a time, and lanes of the
+// Latency-bound on its loads: two pixels of a thread are in flight at a time, and lanes of the
 // same channels (G a power of two) are summed by shuffles before the shared-memory atomics.
+// 65536 pixels, with one, two and four in flight: 32 channels 4.2, 4.1 and 5.7 us, 40 channels
+// 13.6, 13.7 and 18.7, 384 channels 23.4, 20.5 and 25.9: a thread has two or three pixels in all.
 __global__ void __launch_bounds__(512) relu_bias_bwd_kernel(const bf16* __restrict__ out, int o_cs, int o_co,
                                                             bf16* __restrict__ d, int d_cs, int d_co, int C,
                                                             long long P, long long ppb, int relu,
@@ -517,7 +519,7 @@ __global__ void __launch_bounds__(512) relu_bias_bwd_kernel(const bf16* __restri
     __syncthreads();
     const long long p0 = blockIdx.x * ppb, p1 = min(P, p0 + ppb);
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    constexpr int U = 4;
+    constexpr int U = 2;
     if (r < K) {
         for (long long p = p0 + r; p < p1; p += (long long)U * K) {
             uint4 gv[U], ov[U];

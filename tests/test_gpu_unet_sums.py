@@ -28,3 +28,25 @@ def test_weight_gradient(cin, cout, B, H, W, shift):
     ref = torch.stack([dy.double().t() @ v for v in _taps(x, B, H, W, cin)], 1).reshape(-1)
     # FP32 sums of P products in a few hundred partial sums: eps * sqrt(P) of the norm and more
     assert float((dw.double() - ref).norm() / ref.norm()) < 1e-5
+
+
+# channel groups that are powers of two and not, one pixel, remainders of the pixels in flight and
+# of the blocks, channel views; the masked gradient is exact, its sums are of up to 30000 bf16
+# values in FP32 (eps * sqrt(P) of their norm and more)
+@pytest.mark.parametrize("C,P", [(8, 1), (8, 4099), (24, 777), (32, 30011), (40, 13), (96, 5003), (256, 601), (384, 1999),
+                                 (512, 300)])
+@pytest.mark.parametrize("relu", [0, 1])
+def test_relu_and_bias(C, P, relu):
+    import torch
+    from mumax2 import _native as nat
+    g = torch.Generator(device="cuda").manual_seed(C + P)
+    out = torch.randn(P, C + 8, device="cuda", generator=g).bfloat16()
+    d = torch.randn(P, C + 16, device="cuda", generator=g).bfloat16()
+    db = torch.ones(C, device="cuda")
+    want = d.clone()
+    if relu:
+        want[:, 16:] = torch.where(out[:, 8:] > 0, d[:, 16:], torch.zeros_like(d[:, 16:]))
+    nat.check(nat.lib().mm_nn_relu_bias_bwd(_p(out), C + 8, 8, _p(d), C + 16, 16, C, P, relu, _p(db), None))
+    assert torch.equal(d, want)
+    ref = 1 + want[:, 16:].double().sum(0)
+    assert float((db.double() - ref).abs().max()) < 1e-5 * max(1.0, P ** 0.5)
