@@ -23,6 +23,7 @@
 #include "mm_internal.h"
 #include "kernel_view.cuh"
 #include "pdl.cuh"
+#include "tiles.h"
 
 #ifndef MM_RHS_PART
 #define MM_RHS_PART 0
@@ -673,39 +674,11 @@ __host__ __device__ constexpr int xinv4_rpb() {
     return (384 / (3 * FS<M>::P2)) > 0 ? 384 / (3 * FS<M>::P2) : 1;
 }
 
-// Rows and threads per block of the row-shaped passes (C2R + epilogue, stage combine).  A
-// full tile (FLEX = false) is xinv4_rpb rows, a compile-time constant.  A FLEX launch passes
-// its own rows and may have more threads than the row transforms use: the extra ones work on
-// the cells only.
-//  * Grids that fill the GPU with full tiles: the full tile, or half of it (tile -1).
-//    (1024 rows of 1024 cells, 256 full tiles: in finer ones the torque takes 279 us, not 264.)
-//  * Fewer full tiles than SMs: the block's cells, not bandwidth, set the time (a
-//    192-thread block of 8 rows of 128 cells walks 5 cells per thread, one dependent
-//    round trip after the other), so the rows spread over up to two blocks per SM with a
-//    thread per cell (at most 384), at least 128 cells to a block while that leaves one
-//    block per SM.  tile -1: half as many rows.  RK45 step, before and after: 128x128 disk
-//    under Slonczewski torque 268 -> 148 us, 128x32 film 154 -> 107, 512x128 strip 214 -> 157.
-// The row count changes the block decomposition only; every cell's arithmetic is the same.
-struct RowTile {
-    bool flex;
-    int rpb, threads;
-};
+// Rows and threads per block of the four-step row-shaped passes (tiles.h); `fit` is the threads
+// that an SM's registers hold.
 template <int M>
-static RowTile xinv4_shape(int nrows, int n2, int nsim, int tile) {
-    constexpr int R0 = xinv4_rpb<M>(), TR = 3 * FS<M>::P2, SMS = 148;
-    auto up32 = [](long long v) { return (int)((v + 31) / 32 * 32); };
-    const long long rows = (long long)nrows * nsim;
-    if ((long long)((nrows + R0 - 1) / R0) * nsim >= SMS) {
-        if (tile < 0 && R0 >= 2 && (R0 / 2) * TR >= 32) return {true, R0 / 2, up32((R0 / 2) * TR)};
-        return {false, R0, up32(R0 * TR)};
-    }
-    long long rpb = rows / (2 * SMS);
-    const long long fill = std::min<long long>((127 + n2) / n2, rows / SMS);
-    rpb = std::max(rpb, fill);
-    if (tile < 0) rpb /= 2;
-    rpb = std::min<long long>(std::max<long long>(rpb, 1), R0);
-    const long long cells = rpb * n2, turns = (cells + 383) / 384;
-    return {true, (int)rpb, std::max(up32((cells + turns - 1) / turns), up32(rpb * TR))};
+static RowTile xinv4_shape(int nrows, int n2, int nsim, int tile, int fit) {
+    return row_tile(xinv4_rpb<M>(), 3 * FS<M>::P2, nrows, n2, nsim, tile, fit);
 }
 
 // R2C rows from the block's shared-memory lines: float x of the line of (row, c) holds the
@@ -1004,7 +977,8 @@ template <int M>
 static cudaError_t launch_combine_rows_t(const CombineArgs& A, const int n[3], float2* S, int hp, int L1,
                                          long long spec_bstride, const float2* tw, int fwd_mask, int nsim,
                                          cudaStream_t st) {
-    const RowTile tile = xinv4_shape<M>(n[0] * n[1], n[2], nsim, 0);
+    // 63 registers, 103 for rows of more than 512 elements
+    const RowTile tile = xinv4_shape<M>(n[0] * n[1], n[2], nsim, 0, M <= 512 ? 1024 : 608);
     const int RPB = tile.rpb, threads = tile.threads;
     const size_t smem = (size_t)(RPB * 3 * FS<M>::LBUF + FS<M>::TWT + M / 2 + 1) * sizeof(float2);
     const cudaError_t e = allow_smem(combine_rows_kernel<M>, smem);
@@ -1545,7 +1519,9 @@ static cudaError_t launch_xinv4_h(const float2* S, int hp, int L1, const float2*
 template <int M, bool TERMS, bool BATCH, bool FWD>
 static cudaError_t launch_xinv4_f(const float2* S, int hp, int L1, const float2* tw, const EpiArgs& A,
                                   cudaStream_t st, int* nblocks, int nsim, int tile) {
-    const RowTile shape = xinv4_shape<M>(A.P.n[0] * A.P.n[1], A.P.n[2], nsim, tile);
+    // registers: 56 (xinv4_epi_lean3_kernel), at most 80, or for rows of more than 512 elements 145
+    const bool lean3 = !TERMS && !BATCH && !FWD && epilogue_spec(A.P) == SPEC_LEAN;
+    const RowTile shape = xinv4_shape<M>(A.P.n[0] * A.P.n[1], A.P.n[2], nsim, tile, lean3 ? 1152 : M <= 512 ? 800 : 416);
     if (shape.flex) return launch_xinv4_h<M, TERMS, BATCH, true, FWD>(S, hp, L1, tw, A, st, nblocks, nsim, shape);
     return launch_xinv4_h<M, TERMS, BATCH, false, FWD>(S, hp, L1, tw, A, st, nblocks, nsim, shape);
 }

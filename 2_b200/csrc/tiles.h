@@ -38,6 +38,47 @@ inline ColTile col_tiles(size_t line_bytes, int ncols, long long outer) {
 // of 2: 257 -> 305).
 inline int split_columns(int ncols, int nsim) { return (long long)((ncols + 1) / 2) * nsim <= SMS ? 2 : 4; }
 
+// Rows and threads per block of the four-step row-shaped passes (C2R + epilogue, stage combine;
+// rhs.cu).  A full tile (flex = false) is `full` rows of `row_threads` threads each, a
+// compile-time constant of the kernel.  A flex launch passes its own rows and may have more
+// threads than the row transforms use: the extra ones work on the cells only.
+//  * Grids that fill the GPU with full tiles: the full tile, or half of it (tile -1).
+//    (1024 rows of 1024 cells, 256 full tiles: in finer ones the torque takes 279 us, not 264.)
+//  * Fewer full tiles than SMs: the block's cells, not bandwidth, set the time (a
+//    192-thread block of 8 rows of 128 cells walks 5 cells per thread, one dependent
+//    round trip after the other), so the rows spread over up to two blocks per SM with a
+//    thread per cell (at most 384), at least 128 cells to a block while that leaves one
+//    block per SM.  tile -1: half as many rows.  RK45 step, before and after: 128x128 disk
+//    under Slonczewski torque 268 -> 148 us, 128x32 film 154 -> 107, 512x128 strip 214 -> 157.
+//  * But never more blocks than the SMs hold at once (fit: the threads that a kernel's registers
+//    leave an SM), or a few blocks run alone at the end: RK23 step of 512 rows of 1024 cells, 512
+//    blocks at one per SM 339 us, 128 blocks 259; 512 rows of 256 cells 111 -> 96 us, nine
+//    simulations of 128x128 cells 118 -> 89.
+// The row count changes the block decomposition only; every cell's arithmetic is the same.
+struct RowTile {
+    bool flex;
+    int rpb, threads;
+};
+inline RowTile row_tile(int full, int row_threads, int nrows, int n2, int nsim, int tile, int fit) {
+    auto up32 = [](long long v) { return (int)((v + 31) / 32 * 32); };
+    auto blocks = [&](long long rpb) { return (nrows + rpb - 1) / rpb * nsim; };
+    const long long rows = (long long)nrows * nsim;
+    if (blocks(full) >= SMS) {
+        if (tile < 0 && full >= 2 && (full / 2) * row_threads >= 32)
+            return {true, full / 2, up32((full / 2) * row_threads)};
+        return {false, full, up32(full * row_threads)};
+    }
+    long long rpb = std::max(rows / (2 * SMS), std::min<long long>((127 + n2) / n2, rows / SMS));
+    if (tile < 0) rpb /= 2;
+    rpb = std::min<long long>(std::max<long long>(rpb, 1), full);
+    for (;; rpb++) {
+        const long long cells = rpb * n2, turns = (cells + 383) / 384;
+        const int threads = std::max(up32((cells + turns - 1) / turns), up32(rpb * row_threads));
+        if (rpb == full || tile < 0 || blocks(rpb) <= (long long)SMS * std::max(1, fit / threads))
+            return {true, (int)rpb, threads};
+    }
+}
+
 // Which kernel sums a convolution's weight gradient, for `stages` of 64 positions and `tiles` of
 // 32 x 32 channels: the ring of positions, or the one that stages each tap.  The ring takes 7 us
 // however small the sum (its halo, one stage after the other, 9216 reductions a block); the

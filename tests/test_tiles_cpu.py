@@ -47,3 +47,16 @@ def test_small_weight_gradients_stage_each_tap(rule):
     large = [(289, 1), (133, 3), (81, 12), (67, 16), (21, 48), (4225, 64)]
     assert rule(*["wgrad_by_ring(%d, %d)" % v for v in small]) == [0] * len(small)
     assert rule(*["wgrad_by_ring(%d, %d)" % v for v in large]) == [1] * len(large)
+
+
+@pytest.mark.parametrize("full,row_threads", [(16, 24), (8, 48), (4, 96)])
+def test_row_tiles_of_small_grids_run_in_one_wave(rule, full, row_threads):
+    """Fewer full tiles than SMs: every row is covered, a block has 32 to 384 threads and enough of
+    them for its row transforms, and no block waits for another to end."""
+    cases = [(rows, n2, nsim, fit) for rows in (1, 37, 147, 149, 150, 296, 297, 450, 512, 590) for n2 in (8, 100, 256, 1024)
+             for nsim in (1, 3) for fit in (416, 800, 1152) if (rows + full - 1) // full * nsim < 148]
+    got = rule(*["row_tile(%d, %d, %d, %d, %d, 0, %d).%s" % (full, row_threads, r, n, s, f, k)
+                 for r, n, s, f in cases for k in ("rpb", "threads")])
+    for (rows, n2, nsim, fit), rpb, threads in zip(cases, got[::2], got[1::2]):
+        assert 1 <= rpb <= full and 32 <= threads <= 384 and threads % 32 == 0 and threads >= rpb * row_threads
+        assert -(-rows // rpb) * nsim <= 148 * max(1, fit // threads)
