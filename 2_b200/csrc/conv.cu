@@ -613,9 +613,8 @@ __global__ void __launch_bounds__(512) xfwd4_kernel(const float* __restrict__ in
 // put in natural order in shared memory, multiplied by the symmetric kernel there (all
 // three components of a (ky, kx) point meet in one thread), taken back into registers
 // and inverse-transformed; only the rows n < n_in are stored.  ZAX: lines along z of bodies too
-// tall for the register multiply, one (ky, kx tile) per block.  Replaces the Stockham
-// Stockham pass for 2-D films (seven barrier-separated stages per transform and
-// component there, two barriers per transform here).
+// tall for the register multiply, one (ky, kx tile) per block.  Two barriers per transform,
+// each of full length, the padding's zeros included.
 template <int L, int TC, bool ZAX>
 __global__ void __launch_bounds__(384) colmul4_kernel(float2* __restrict__ S, KernelView K, int ncols,
                                                       long long comp_stride, long long outer_stride,
@@ -959,12 +958,7 @@ static cudaError_t launch_colmul4_t(float2* S, const KernelView& K, int ncols, l
                                     long long line_stride, int n_in, float scale, const float2* tw,
                                     const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
                                     long long sim_stride, const float* sim_scale, int tile) {
-    // single small films of up to 64 rows: fewer columns per block while the blocks leave SMs
-    // idle (a 128x32 film has 129 columns, 17 blocks of the default 8).  Longer columns keep
-    // their tile: 48-thread blocks of one 256-point column take 11.1 us, 192-thread ones 10.0.
-    int shift = tile;
-    const long long cols = (long long)ncols * nsim;
-    while (L <= 128 && shift > -3 && cols < 148LL * (64 / FS<L>::P2 >> -std::min(shift, 0))) shift--;
+    const int shift = colmul4_shift(L, FS<L>::P2, (long long)ncols * nsim, tile);
 #define GO(sh)                                                                                                  \
     return launch_colmul4_s<L, sh, false>(S, K, ncols, 1, comp_stride, 0, line_stride, n_in, scale, tw, ctl,    \
                                           skip_retry, st, nsim, sim_stride, sim_scale)

@@ -38,6 +38,17 @@ inline ColTile col_tiles(size_t line_bytes, int ncols, long long outer) {
 // of 2: 257 -> 305).
 inline int split_columns(int ncols, int nsim) { return (long long)((ncols + 1) / 2) * nsim <= SMS ? 2 : 4; }
 
+// Columns per block of the four-step multiply (colmul4_kernel), as a shift of its default 64 / P2
+// (P2 threads per column): the default, on grids of columns of up to 128 points as much narrower
+// (an eighth at most) as leaves one block per SM; then half or double that (tile -1, +1).  A film
+// of 128x32 cells has 129 columns, 17 blocks of the default 8.  Longer columns keep their tile:
+// 48-thread blocks of one 256-point column take 11.1 us, 192-thread ones 10.0.
+inline int colmul4_shift(int L, int P2, long long cols, int tile) {
+    int shift = 0;
+    while (L <= 128 && shift > -3 && cols < (long long)SMS * (64 / P2 >> -shift)) shift--;
+    return std::max(-3, std::min(1, shift + tile));
+}
+
 // Rows and threads per block of the four-step row-shaped passes (C2R + epilogue, stage combine;
 // rhs.cu).  A full tile (flex = false) is `full` rows of `row_threads` threads each, a
 // compile-time constant of the kernel.  A flex launch passes its own rows and may have more

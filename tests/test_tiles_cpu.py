@@ -60,3 +60,11 @@ def test_row_tiles_of_small_grids_run_in_one_wave(rule, full, row_threads):
     for (rows, n2, nsim, fit), rpb, threads in zip(cases, got[::2], got[1::2]):
         assert 1 <= rpb <= full and 32 <= threads <= 384 and threads % 32 == 0 and threads >= rpb * row_threads
         assert -(-rows // rpb) * nsim <= 148 * max(1, fit // threads)
+
+
+def test_multiply_tiles_stay_apart(rule):
+    """Narrowed columns of small films still halve and double by the plan's tile."""
+    assert rule(*["colmul4_shift(64, 8, 257, %d)" % t for t in (-1, 0, 1)]) == [-3, -3, -2]
+    assert rule(*["colmul4_shift(64, 8, 513, %d)" % t for t in (-1, 0, 1)]) == [-3, -2, -1]
+    assert rule(*["colmul4_shift(64, 8, 100000, %d)" % t for t in (-1, 0, 1)]) == [-1, 0, 1]
+    assert rule(*["colmul4_shift(256, 16, 129, %d)" % t for t in (-1, 0, 1)]) == [-1, 0, 1]
