@@ -71,3 +71,29 @@ def test_batched(n):
     for b in range(sims):
         assert rel_err(got[b], _field64(g, n, (0, 0, 0), states[b], masks[b], msat[b])) < 1e-6
     g.close()
+
+
+def test_finished_simulations_in_a_group():
+    """A block of the z multiply that does several simulations passes over those that have
+    finished: each one's steps and state are those of its own plan."""
+    from mumax2 import Plan
+    n, sims = (4, 128, 128), 18
+    prob = _prob(n)
+    thr = np.where(np.arange(sims) % 3 == 1, 1e15, 1e-3)   # every third one stops at once
+    msat = [8e5 * (1 - 0.02 * b) for b in range(sims)]
+    states = [rand_m(n, seed=b).astype(np.float32) for b in range(sims)]
+    g = Plan(prob, sims=[dict(prob, msat=v) for v in msat])
+    g.solver("rk23", dt=1e-15, maxerr=1e-5)
+    g.set_state(np.concatenate(states))
+    g.batch_run_until_maxtorque(thr, max_steps=5)
+    got, stats = g.get_state().reshape(sims, -1), g.batch_stats()
+    assert len({s["step"] for s in stats}) == 2
+    for b in range(0, sims, 5):
+        one = Plan(dict(prob, msat=msat[b]))
+        one.solver("rk23", dt=1e-15, maxerr=1e-5)
+        one.set_state(states[b])
+        one.run_until_maxtorque(thr[b], max_steps=5)
+        assert one.stats()["step"] == stats[b]["step"]
+        assert np.abs(got[b] - one.get_state()).max() < 2e-6   # rounding of the scaled spectrum, a few steps
+        one.close()
+    g.close()

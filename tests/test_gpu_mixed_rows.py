@@ -32,3 +32,34 @@ def test_row_output_batched(monkeypatch):
     _, sims, _ = W.relax_set(5, seed=3)
     m0 = np.concatenate([rand_m(n, seed=s) for s in range(5)])
     _compare(monkeypatch, prob, m0, "rk23", 10, sims=sims, dt=1e-14, maxerr=1e-5)
+
+
+def test_row_output_demag_exchange(monkeypatch):
+    """The exchange inside the kernel: the rows are of the state, not of Ms times the state."""
+    import oracle as O
+    n = (2, 12, 20)
+    mask = np.random.default_rng(4).uniform(0.5, 1.0, size=n[0] * n[1] * n[2]).astype(np.float32)
+    prob = O.full_desc(n=n, cell=(3e-9, 4e-9, 4e-9), demag=1, exchange=0, zeeman=1, msat=8e5, aex=1.3e-11, alpha=0.1,
+                       bext=(0.0, 0.01, 0.02), demag_exchange=1, demag_accuracy=2, masks={"msat": mask})
+    _compare(monkeypatch, prob, rand_m(n, seed=8), "rk23", 10, masks={"msat": mask}, dt=1e-14, maxerr=1e-5)
+
+
+@pytest.mark.parametrize("solver", ["rk23", "rk12"])
+def test_row_output_time_table(monkeypatch, solver):
+    """A field table: the staged scalars of a single plan, at each stage's own time."""
+    from mumax2 import Plan
+    n = (1, 18, 44)
+    prob = dict(n=n, cell=(3e-9, 4e-9, 4e-9), demag=1, exchange=1, zeeman=1, msat=8e5, aex=1.3e-11, alpha=0.1,
+                bext=(0.0, 1.0, 1.0), demag_accuracy=2)
+    out = []
+    for rows in ("0", "1"):
+        monkeypatch.setenv("MM_EPI_R2C", rows)
+        p = Plan(prob)
+        p.solver(solver, dt=1e-13, maxerr=1e-5)
+        p.set_state(rand_m(n, seed=6))
+        p.set_table("bext", [0.0, 2e-13, 1e-12, 1e-9], [(0, 0, 0), (0, 0.1, 0.3), (0.2, 0.0, 0.1), (0, 0, 0)])
+        p.steps(8)
+        out.append(p.get_state())
+        p.close()
+    assert np.array_equal(out[0], out[1])
+    assert not np.array_equal(out[0], rand_m(n, seed=6).astype(np.float32))

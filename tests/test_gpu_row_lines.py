@@ -1,10 +1,13 @@
 """Rows whose lengths are not powers of two, at every number of lines that a block takes: 1, 2, 4,
 8 and 16 rows in the row pass, 3, 6 and 15 lines in the epilogue, with and without a radix above
-10; field and torque against the FP64 oracle, and the epilogue's row output against the row pass."""
+10; the field against the convolution with the plan's own kernel in FP64, and the epilogue's row
+output against the row pass."""
+import numpy as np
 import pytest
 
 from helpers import rand_m, rel_err, to_np
 from test_gpu_epi_r2c import _compare
+from test_gpu_long_columns import _field64
 
 pytestmark = pytest.mark.gpu
 
@@ -18,16 +21,14 @@ def _prob(n):
                        demag_accuracy=1)
 
 
-# the bounds of test_gpu_sizes: FP32 transforms of up to 4096 points, eps * log2(L) each way
+# the bound of test_gpu_sizes: FP32 transforms of up to 4096 points, eps * log2(L) each way
 @pytest.mark.parametrize("n", SIZES)
-def test_field_and_torque(n):
-    import oracle as O
+def test_field(n):
     from mumax2 import Plan
-    prob = _prob(n)
-    o, g = O.Oracle(prob), Plan(prob)
-    m = rand_m(n, seed=sum(n))
-    assert rel_err(to_np(g.fields(m)["demag"]), o.fields(m)["demag"]) < 1e-6
-    assert rel_err(to_np(g.torque(m)[0]), o.torque(m)[0]) < 2e-6
+    g = Plan(_prob(n))
+    m = rand_m(n, seed=sum(n)).astype(np.float32)
+    want = _field64(g, n, (0, 0, 0), m, np.ones(n[0] * n[1] * n[2], np.float32), 8e5)
+    assert rel_err(to_np(g.fields(m)["demag"]), want) < 1e-6
     g.close()
 
 
