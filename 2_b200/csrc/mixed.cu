@@ -91,18 +91,6 @@ bool mr_tables(int L, const float2** tf, const double2** td) {
     return false;
 }
 
-template <typename V> static const V* pick_table(const float2* f, const double2* d);
-template <> const float2* pick_table<float2>(const float2* f, const double2*) { return f; }
-template <> const double2* pick_table<double2>(const float2*, const double2* d) { return d; }
-
-template <typename V> static bool table_of(int L, const V** out) {
-    const float2* f = nullptr;
-    const double2* d = nullptr;
-    if (!mr_tables(L, &f, &d)) return false;
-    *out = pick_table<V>(f, d);
-    return true;
-}
-
 // ---------------------------------------------------------------- R2C row pass
 // As xfwd_kernel: rows r = (c*Z + z)*Y + y of n_in reals (times the mask), zero-padded to
 // 2M, packed as z[e] = x[2e] + i x[2e+1], transformed (length M) and post-processed into
@@ -171,7 +159,7 @@ cudaError_t launch_mr_xfwd(int M, const S* in, PP pp, const float* mask, V* out,
                            int nsim, long long in_bstride, long long out_bstride, long long mask_bstride) {
     MrLine f;
     const V *twM = nullptr, *tw2M = nullptr;
-    if (!mr_factor(M, &f) || !table_of<V>(M, &twM) || !table_of<V>(2 * M, &tw2M)) return cudaErrorInvalidValue;
+    if (!mr_factor(M, &f) || !mr_tables(M, nullptr, &twM) || !mr_tables(2 * M, nullptr, &tw2M)) return cudaErrorInvalidValue;
     const int nt = mr_row_threads(M);
     const int rpb = 256 / nt;
     const size_t smem = (size_t)rpb * 2 * M * sizeof(V);
@@ -253,7 +241,7 @@ cudaError_t launch_mr_xfwd<float2, float>(int M, const float* in, PP pp, const f
                                           long long out_bstride, long long mask_bstride) {
     ColPlan P;
     const float2 *twM = nullptr, *tw2M = nullptr;
-    if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !table_of<float2>(2 * M, &tw2M)) return cudaErrorInvalidValue;
+    if (!col_plan(M, false, 10, 10, nullptr, &P, &twM) || !mr_tables(2 * M, &tw2M, nullptr)) return cudaErrorInvalidValue;
     const int tc = rows_per_block(M, (long long)nrows * nsim);
     set_lines(&P, tc);
     const size_t smem = lines_smem(M, tc);
@@ -317,7 +305,7 @@ cudaError_t launch_mr_colfft(int L, int sign, V* S, int ncols, int nouter, long 
                              cudaStream_t st, int nsim, long long sim_stride) {
     MrLine f;
     const V* tw = nullptr;
-    if (!mr_factor(L, &f) || !table_of<V>(L, &tw)) return cudaErrorInvalidValue;
+    if (!mr_factor(L, &f) || !mr_tables(L, nullptr, &tw)) return cudaErrorInvalidValue;
     const int TC = mr_cols(L, 2, sizeof(V));
     const size_t smem = (size_t)2 * TC * L * sizeof(V);
     const int ntiles = (ncols + TC - 1) / TC;

@@ -41,9 +41,6 @@ bool mr_tables(int L, const float2** tf, const double2** td);
 // Whether the power-of-two passes serve length L (else the mixed-radix ones do).
 inline bool mr_pow2(int L) { return L > 0 && (L & (L - 1)) == 0 && L <= MR_MAXL; }
 
-template <typename V> struct MrTab;
-template <> struct MrTab<float2> { typedef const float2* type; };
-template <> struct MrTab<double2> { typedef const double2* type; };
 
 // exp(SIGN 2 pi i t / L) from the table (t < L)
 template <int SIGN, typename V>
