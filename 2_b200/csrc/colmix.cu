@@ -248,8 +248,9 @@ __global__ void __launch_bounds__(512) colmix_fft_kernel(float2* __restrict__ S,
 }
 
 // Three components per column: forward, symmetric kernel multiply, inverse.  kaxis 0: lines
-// along z (ky = o), 1: along y (kz = 0).  Bound by registers and shared memory (few warps);
-// lengths that are powers of two have faster four-step passes (conv.cu).
+// along z (ky = o), 1: along y (kz = 0).  Bound by registers and shared memory (few warps: one
+// block of 512 threads per SM or two of 256); lengths that are powers of two up to 1024 have faster
+// four-step passes (conv.cu).
 __global__ void __launch_bounds__(512) colmix_mul_kernel(float2* __restrict__ S, KernelView K, int ncols,
                                                          long long comp_stride, long long outer_stride, long long ls,
                                                          int n_in, int kaxis, float scale, const __grid_constant__ ColPlan P,

@@ -460,7 +460,10 @@ cudaError_t launch_zmul_reg(int P, float2* S, const KernelView& K, int L1, int h
 #define X(p, f) case p: return f<p>(S, K, L1, h, hp, comp_stride, zstride, scale, tw, tws, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
         // two lanes per column up to P = 15 (P = 3, 150x75x3 body: 5.5 us, where the columns in
         // shared memory took 46; measured besides: P = 4, 128x128x4 ensemble class
-        // 1073 -> 1012 us; P = 8, 8x128x128 film 11.8 -> 11.0 us), four at P = 16
+        // 1073 -> 1012 us; P = 8, 8x128x128 film 11.8 -> 11.0 us), four at P = 16.  P = 9..15 take
+        // 168-255 registers and spill 48-160 bytes from 12 on in a batch; 16 simulations of Px128x128:
+        // P = 8 70 us, 10 110, 11 170, 15 250, 16 (four lanes) 210.  In columns in shared memory a
+        // torque of Px128x128 took 140, 130 and 163 us for P = 9, 12 and 15; now 50, 58 and 64.
         X(1, launch_zmul_reg_t) X(2, launch_zmul_reg_t) X(3, launch_zmul_reg_t) X(4, launch_zmul_reg_t)
         X(5, launch_zmul_reg_t) X(6, launch_zmul_reg_t) X(7, launch_zmul_reg_t) X(8, launch_zmul_reg_t)
         X(9, launch_zmul_reg_t) X(10, launch_zmul_reg_t) X(11, launch_zmul_reg_t) X(12, launch_zmul_reg_t)
@@ -987,7 +990,10 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
         }
     }
     if (kaxis == 0) {
-        // tall bodies: the four-step pass along z (64^3 cells: 45 us; Stockham stages 81)
+        // tall bodies: the four-step pass along z (64^3 cells: 45 us; Stockham stages 81).  The other
+        // lengths, RK23 step with Stockham stages and now: 32, 128 and 256 layers of 32x32 cells 116 ->
+        // 75, 242 -> 139 and 319 -> 219 us; periodic, 8, 16 and 512 layers 107 -> 73, 112 -> 77 (64x64)
+        // and 189 -> 118 (16x16)
         switch (L) {
 #define X(l) case l: return launch_colmul4_s<l, 0, true>(S, K, ncols, nouter, comp_stride, outer_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st, nsim, sim_stride, sim_scale);
             X(8) X(16) X(32) X(64) X(128) X(256) X(512)

@@ -569,7 +569,7 @@ __device__ __forceinline__ const SimScalars& pick_scalars(const SimScalars& stag
 // even x, imaginary part for odd x) of shared-memory line (lrow*3 + c), stride LS.
 // TRANSP: the lines side by side, element e of line l at sm[e * LS + l].
 // FWD: float x of line (lrow, c) then takes the cell's next state (times the Msat mask
-// when A.fwd_mask) for the R2C rows of the next evaluation (four-step lines only).
+// when A.fwd_mask) for the R2C rows of the next evaluation (not PADDED lines).
 template <bool TERMS, bool PADDED, bool BATCH, bool FWD = false, int SPEC = 0, bool TRANSP = false>
 __device__ __forceinline__ void epilogue_rows(const EpiArgs& A, const SimScalars& S0, const float2* sm, int LS,
                                               int row0, int nrow_here) {
@@ -580,7 +580,7 @@ __device__ __forceinline__ void epilogue_rows(const EpiArgs& A, const SimScalars
     // the reference (256 films, six RK23 steps 2660 us; by value 2790, with spills).
     typedef typename std::conditional<BATCH && (SPEC & SPEC_NOMASK) != 0, const SimScalars, const SimScalars&>::type Sc;
     Sc S = S0;
-    static_assert(!(FWD && (PADDED || TERMS)), "row output: four-step lines, no per-term outputs");
+    static_assert(!(FWD && (PADDED || TERMS)), "row output: four-step or transposed lines, no per-term outputs");
     const int n1 = A.P.n[1], n2 = A.P.n[2];
     const DevCtl* ctl;
     ResolvedOp r;

@@ -42,7 +42,8 @@ inline int split_columns(int ncols, int nsim) { return (long long)((ncols + 1) /
 // (P2 threads per column): the default, on grids of columns of up to 128 points as much narrower
 // (an eighth at most) as leaves one block per SM; then half or double that (tile -1, +1).  A film
 // of 128x32 cells has 129 columns, 17 blocks of the default 8.  Longer columns keep their tile:
-// 48-thread blocks of one 256-point column take 11.1 us, 192-thread ones 10.0.
+// 48-thread blocks of one 256-point column take 11.1 us, 192-thread ones 10.0.  (Within the narrowed
+// ones it matters little: films of 32 rows 8.6 us and of 64 rows 10.6 us at -1, 0 and +1.)
 inline int colmul4_shift(int L, int P2, long long cols, int tile) {
     int shift = 0;
     while (L <= 128 && shift > -3 && cols < (long long)SMS * (64 / P2 >> -shift)) shift--;
@@ -54,7 +55,8 @@ inline int colmul4_shift(int L, int P2, long long cols, int tile) {
 // compile-time constant of the kernel.  A flex launch passes its own rows and may have more
 // threads than the row transforms use: the extra ones work on the cells only.
 //  * Grids that fill the GPU with full tiles: the full tile, or half of it (tile -1).
-//    (1024 rows of 1024 cells, 256 full tiles: in finer ones the torque takes 279 us, not 264.)
+//    (1024 rows of 1024 cells, 256 full tiles: in finer ones the torque took 279 us, not 264;
+//    both would be 70 less with the columns of today.)
 //  * Fewer full tiles than SMs: the block's cells, not bandwidth, set the time (a
 //    192-thread block of 8 rows of 128 cells walks 5 cells per thread, one dependent
 //    round trip after the other), so the rows spread over up to two blocks per SM with a

@@ -978,7 +978,7 @@ __device__ __forceinline__ bool mbar_wait(unsigned addr, unsigned parity, long l
 __host__ __device__ constexpr int band_max(int T) { return 128 * T + 2 * 257 + 2; }  // widths up to 256
 
 // A block computes T consecutive tiles of 128 positions, each in its own N TMEM columns, from
-// one band and one copy of the weights: the W+2 halo on both sides of the band (130 positions
+// one band and one copy of the weights: the W+2 halo on both sides of the band (132 positions
 // beside 128 at W = 64) and the block's set-up are paid once per T tiles.  32 -> 32 channels on
 // 64 images of 64x64: 49.5 -> 33 us (34 MB of traffic; bound by the latency of its few slices).
 template <int N, int ST, int T>
