@@ -159,8 +159,12 @@ class UNet:
         nw = [c[4] * 9 * c[2] for c in CONVS]
         cin_t = [((c[4] + 15) // 16) * 16 for c in CONVS]
         nt = [c[2] * 9 * t for c, t in zip(CONVS, cin_t)]
-        host = np.concatenate([params[c[0]][k].ravel() for k in (0, 1) for c in CONVS]).astype(np.float32)
-        flat = {"w": torch.tensor(host, device=self.device)}
+        flat = {"w": torch.cat([torch.as_tensor(params[c[0]][k], dtype=torch.float32, device=self.device).reshape(-1)
+                                for k in (0, 1) for c in CONVS])}
+        for c, n in zip(CONVS, nw):
+            got = tuple(int(np.prod(np.shape(v))) for v in params[c[0]])
+            if got != (n, c[4]):
+                raise ValueError("layer %s: %d weights and %d biases, expected %d and %d" % ((c[0],) + got + (n, c[4])))
         for k in ("g", "m", "v"):
             flat[k] = torch.zeros_like(flat["w"])
         flat["wb"] = flat["w"][:sum(nw)].to(bf)

@@ -50,3 +50,25 @@ def test_relu_and_bias(C, P, relu):
     assert torch.equal(d, want)
     ref = 1 + want[:, 16:].double().sum(0)
     assert float((db.double() - ref).abs().max()) < 1e-5 * max(1.0, P ** 0.5)
+
+
+def test_parameters_of_another_network():
+    """A network takes another one's device tensors, arrays of any float type and plain lists, and
+    refuses layers of other sizes."""
+    import numpy as np
+    import torch
+    from mumax2 import unet as U
+    a = U.UNet(1, H=16, W=16, seed=5)
+    forms = {"tensors": lambda t: t, "doubles": lambda t: t.cpu().numpy().astype(np.float64), "lists": lambda t: t.tolist()}
+    for form in forms.values():
+        b = U.UNet(2, H=16, W=16, params={n: (form(d["w"]), form(d["b"])) for n, d in a.p.items()})
+        for n, d in a.p.items():
+            for k in ("w", "b", "wb", "wt"):
+                assert torch.equal(d[k], b.p[n][k]), (n, k)
+    b.p["out"]["w"].add_(1.0)   # the copies are the network's own
+    assert not torch.equal(a.p["out"]["w"], b.p["out"]["w"])
+    short = {n: (d["w"], d["b"]) for n, d in a.p.items()}
+    first = next(iter(short))
+    short[first] = (short[first][0][:-1], short[first][1])
+    with pytest.raises(ValueError, match=first):
+        U.UNet(1, H=16, W=16, params=short)
