@@ -627,9 +627,10 @@ __device__ __forceinline__ void epilogue_rows(const EpiArgs& A, const SimScalars
     block_reduce_publish(tr, A.op, const_cast<DevCtl*>(ctl), A.tq_out, A.red);
 }
 
-// Stockham variant (any power-of-two M up to 2048; single-simulation plans)
+// Stockham variant (any power-of-two M up to 2048, whose one row per block takes 768 threads;
+// single-simulation plans)
 template <int M, bool TERMS>
-__global__ void __launch_bounds__(512) xinv_epi_kernel(const float2* __restrict__ S, int hp, int L1,
+__global__ void __launch_bounds__(3 * tpl(M) > 512 ? 3 * tpl(M) : 512) xinv_epi_kernel(const float2* __restrict__ S, int hp, int L1,
                                                        const float2* __restrict__ tw, EpiArgs A) {
     const DevCtl* ctl = A.ctl ? A.ctl + blockIdx.y : nullptr;
     if (skip_eval(ctl, A.skip_retry)) return;
