@@ -191,6 +191,48 @@ __global__ void colfft_kernel(V* __restrict__ S, int ncols, long long outer_stri
     tile_store<L, TC, V>(sm, base, line_stride, n_out, nh, 0);
 }
 
+// Three components of one column per block: forward, H_d = sum_s Khat_sd M_s (symmetric, real;
+// kz = 0), inverse, each component by the whole block.  For columns of 2048 and 4096 points that
+// are not zero-padded, on films too narrow to fill the GPU (line_columns in tiles.h); bound by
+// its chain of barriers.
+template <int L>
+__global__ void __launch_bounds__(tpl(L)) colmul_line_kernel(float2* __restrict__ S, KernelView K,
+                                                             long long comp_stride, long long line_stride, int n_in,
+                                                             float scale, const float2* __restrict__ tw,
+                                                             const DevCtl* ctl, int skip_retry, long long sim_stride,
+                                                             const float* __restrict__ sim_scale) {
+    if (ctl) ctl += blockIdx.y;
+    if (conv_skip(ctl, skip_retry)) return;
+    S += blockIdx.y * sim_stride + blockIdx.x;
+    if (sim_scale) scale = sim_scale[blockIdx.y];
+    constexpr int LL = line_len(L);
+    extern __shared__ unsigned char smem_raw[];
+    float2* sm = reinterpret_cast<float2*>(smem_raw);
+#pragma unroll 1
+    for (int c = 0; c < 3; c++) tile_load<L, 1, float2>(sm, S + c * comp_stride, line_stride, n_in, 1, c, true);
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < 3; c++) fft_line<L, -1, float2>(sm + c * LL, threadIdx.x, true, tw);
+    for (int ky = threadIdx.x; ky < L; ky += blockDim.x) {
+        float kk[6];
+        kernel_at(K, 0, ky, blockIdx.x, kk);
+        float2* l0 = sm + padx(ky);
+        const float2 m0 = l0[0], m1 = l0[LL], m2 = l0[2 * LL];
+        // q: 0 xx, 1 yy, 2 zz, 3 yz, 4 xz, 5 xy
+        l0[0] = make_float2(scale * (kk[0] * m0.x + kk[5] * m1.x + kk[4] * m2.x),
+                            scale * (kk[0] * m0.y + kk[5] * m1.y + kk[4] * m2.y));
+        l0[LL] = make_float2(scale * (kk[5] * m0.x + kk[1] * m1.x + kk[3] * m2.x),
+                             scale * (kk[5] * m0.y + kk[1] * m1.y + kk[3] * m2.y));
+        l0[2 * LL] = make_float2(scale * (kk[4] * m0.x + kk[3] * m1.x + kk[2] * m2.x),
+                                 scale * (kk[4] * m0.y + kk[3] * m1.y + kk[2] * m2.y));
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < 3; c++) fft_line<L, +1, float2>(sm + c * LL, threadIdx.x, true, tw);
+#pragma unroll 1
+    for (int c = 0; c < 3; c++) tile_store<L, 1, float2>(sm, S + c * comp_stride, line_stride, n_in, 1, c);
+}
+
 // ---------------------------------------------------------------- register z-multiply
 // The 3-D z pass without shared memory.  With the z direction zero-padded to
 // L0 = 2P (P = N0 non-zero planes), the forward transform splits into its even and odd
@@ -891,6 +933,16 @@ cudaError_t launch_colfft(int L, int sign, V* S, int ncols, int nouter, long lon
         }
     }
     if constexpr (sizeof(V) == 8) {
+        if (line_columns(L, (long long)ncols * nouter * nsim)) {
+#define GO(l, s) return launch_colfft_t<l, s, V>(S, ncols, nouter, outer_stride, line_stride, n_in, n_out, tw, ctl, skip_retry, st, nsim, sim_stride)
+            if (L == 2048) {
+                if (sign < 0) GO(2048, -1);
+                GO(2048, 1);
+            }
+            if (sign < 0) GO(4096, -1);
+            GO(4096, 1);
+#undef GO
+        }
         return launch_colmix_fft(L, sign, S, ncols, nouter, outer_stride, line_stride, n_in, n_out, tw, ctl,
                                  skip_retry, st, nsim, sim_stride);
     } else if (sign < 0) {
@@ -975,6 +1027,22 @@ static cudaError_t launch_colmul4_t(float2* S, const KernelView& K, int ncols, l
 #undef GO
 }
 
+template <int L>
+static cudaError_t launch_colmul_line(float2* S, const KernelView& K, int ncols, long long comp_stride,
+                                      long long line_stride, int n_in, float scale, const float2* tw,
+                                      const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
+                                      long long sim_stride, const float* sim_scale) {
+    const size_t smem = 3 * line_len(L) * sizeof(float2);
+    const cudaError_t e = allow_smem(colmul_line_kernel<L>, smem);
+    if (e != cudaSuccess) return e;
+    // Launched the ordinary way: with one block per SM, the ones that start early gather on the SMs
+    // that become free first (RK23 step of periodic 2048x128 cells 192 us, so 141; 4096x128 252 and
+    // 237).
+    colmul_line_kernel<L><<<dim3((unsigned)ncols, (unsigned)nsim), tpl(L), smem, st>>>(
+        S, K, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, sim_stride, sim_scale);
+    return cudaGetLastError();
+}
+
 cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int nouter, long long comp_stride,
                           long long outer_stride, long long line_stride, int n_in, int kaxis, float scale,
                           const float2* tw, const DevCtl* ctl, int skip_retry, cudaStream_t st, int nsim,
@@ -1000,6 +1068,13 @@ cudaError_t launch_colmul(int L, float2* S, const KernelView& K, int ncols, int 
 #undef X
             default: break;
         }
+    }
+    if (kaxis == 1 && nouter == 1 && 2 * n_in > L && line_multiply(L, (long long)ncols * nsim)) {
+        if (L == 2048)
+            return launch_colmul_line<2048>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st,
+                                            nsim, sim_stride, sim_scale);
+        return launch_colmul_line<4096>(S, K, ncols, comp_stride, line_stride, n_in, scale, tw, ctl, skip_retry, st,
+                                        nsim, sim_stride, sim_scale);
     }
     if (kaxis == 1 && nouter == 1 && L == 2048 && 2 * n_in <= L) {
         if (split_columns(ncols, nsim) == 2)

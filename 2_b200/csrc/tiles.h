@@ -33,6 +33,15 @@ inline ColTile col_tiles(size_t line_bytes, int ncols, long long outer) {
     return {tc, alone ? 512 : 256};
 }
 
+// Columns of 2048 and 4096 points that few blocks work on take the Stockham stages, a column's 256
+// or 512 threads on one stage after the other, instead of the in-place columns: the transforms
+// while there are at most 3072 points per SM, the multiply of columns without padding while there
+// is at most one per SM.  Torque, in place and with these: 2x1024x32 cells 53.6 and 45.5 us, 4x1024x32
+// (396 columns) 60.2 and 62.7; 2x2048x16 56.7 and 49.0, 2x2048x32 (198) 65.9 and 69.8; periodic
+// 4096x64 82.4 and 68.1, 4096x256 137.7 and 164.5.
+inline bool line_columns(int L, long long cols) { return (L == 2048 || L == 4096) && cols * L <= SMS * 3072LL; }
+inline bool line_multiply(int L, long long cols) { return (L == 2048 || L == 4096) && cols <= SMS; }
+
 // Columns per block of the parity-split multiply of 2048-point columns: 4, or 2 by the same rule
 // (1024 rows of 64 cells 155 -> 126 us a step, of 256 cells 214 -> 186; of 512 cells, 257 blocks
 // of 2: 257 -> 305).

@@ -44,7 +44,10 @@ def _field64(plan, n, pbc, m, mask, msat):
                                    ((1, 1000, 1024), (0, 0, 0)), ((1, 1200, 6), (0, 0, 0)), ((1, 1300, 150), (0, 0, 0)),
                                    ((1, 2048, 4), (0, 0, 0)), ((1, 2048, 75), (0, 0, 0)), ((1, 2000, 192), (0, 0, 0)),
                                    ((1, 2048, 6), (0, 1, 0)), ((1, 1024, 8), (0, 1, 0)), ((2, 1024, 8), (0, 0, 0)),
-                                   ((3, 1200, 6), (0, 0, 0)), ((32, 24, 30), (0, 0, 0)), ((128, 6, 10), (0, 0, 0)),
+                                   ((3, 1200, 6), (0, 0, 0)),
+                                   ((4, 1024, 32), (0, 0, 0)), ((2, 2048, 5), (0, 0, 0)), ((2, 2048, 32), (0, 0, 0)),
+                                   ((2, 2048, 6), (0, 1, 0)), ((2, 4096, 5), (1, 1, 0)), ((1, 4096, 6), (0, 1, 0)),
+                                   ((1, 4096, 150), (0, 1, 0)), ((1, 2048, 150), (0, 1, 0)), ((32, 24, 30), (0, 0, 0)), ((128, 6, 10), (0, 0, 0)),
                                    ((256, 4, 6), (0, 0, 0)), ((8, 20, 12), (1, 0, 0)), ((16, 12, 20), (1, 0, 0)),
                                    ((64, 6, 8), (1, 1, 0)), ((18, 30, 40), (0, 0, 0)), ((20, 8, 6), (1, 0, 1))])
 def test_field(n, pbc):
@@ -56,20 +59,21 @@ def test_field(n, pbc):
     g.close()
 
 
-@pytest.mark.parametrize("n", [(1, 1024, 8), (1, 1024, 75), (1, 1200, 8), (4, 128, 128), (3, 100, 121)])
-def test_batched(n):
+@pytest.mark.parametrize("n,along_y", [((1, 1024, 8), 0), ((1, 1024, 75), 0), ((1, 1200, 8), 0), ((4, 128, 128), 0), ((3, 100, 121), 0),
+                                   ((1, 2048, 6), 1), ((2, 2048, 4), 1)])
+def test_batched(n, along_y):
     """Every simulation of a batch with its own material, mask and state.  The bodies fill the GPU,
     so a block of their z multiply does several simulations, the last one fewer."""
     from mumax2 import Plan
-    N, sims = n[0] * n[1] * n[2], 21
-    prob = _prob(n)
+    N, sims, pbc = n[0] * n[1] * n[2], 21, (0, along_y, 0)
+    prob = _prob(n, pbc)
     msat = [8e5 * (1 - 0.02 * b) for b in range(sims)]
     masks = [np.random.default_rng(b).uniform(0.4, 1.0, N).astype(np.float32) for b in range(sims)]
     states = [rand_m(n, seed=b).astype(np.float32) for b in range(sims)]
     g = Plan(prob, masks={"msat": np.concatenate(masks)}, sims=[dict(prob, msat=v) for v in msat], masks_per_sim=True)
     got = to_np(g.fields(np.concatenate(states))["demag"]).reshape(sims, 3 * N)
     for b in range(sims):
-        assert rel_err(got[b], _field64(g, n, (0, 0, 0), states[b], masks[b], msat[b])) < 1e-6
+        assert rel_err(got[b], _field64(g, n, pbc, states[b], masks[b], msat[b])) < 1e-6
     g.close()
 
 

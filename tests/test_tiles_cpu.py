@@ -42,6 +42,13 @@ def test_split_columns(rule):
         [2, 2, 4, 4]
 
 
+def test_few_long_columns_take_their_own_stages(rule):
+    assert rule("line_columns(2048, 198)", "line_columns(2048, 390)", "line_columns(4096, 102)",
+                "line_columns(4096, 198)", "line_columns(1024, 8)", "line_columns(1200, 8)") == [1, 0, 1, 0, 0, 0]
+    assert rule("line_multiply(4096, 129)", "line_multiply(4096, 257)", "line_multiply(2048, 65)",
+                "line_multiply(3000, 9)") == [1, 0, 1, 0]
+
+
 def test_small_weight_gradients_stage_each_tap(rule):
     small = [(1, 1), (5, 1), (81, 1), (162, 1), (81, 4), (18, 16), (10, 48), (9, 48)]
     large = [(289, 1), (133, 3), (81, 12), (67, 16), (21, 48), (4225, 64)]
