@@ -1,4 +1,4 @@
-"""Rows of 1025 to 2048 cells that transform at 4096 points, and their time steps, against the FP64
+"""Rows of 2048 cells, which transform at 4096 points: field, torque and time steps against the FP64
 oracle."""
 import numpy as np
 import pytest
